@@ -54,7 +54,7 @@ def listed():
         dict(name="solver3d_det_300k", kind="solver", dim=3, n=300_000, res=96, dtype="f32", substeps=20,
              deterministic=True),
         # the batched workload: 256 scenes of 2k to 64k particles
-        dict(name="batch2d_256", kind="batch2d", scenes=256, n_lo=2048, n_hi=65536, dtype="f32", substeps=20),
+        dict(name="batch2d_256", kind="batch2d", scenes=256, n_lo=2048, n_hi=65536, dtype="f32", substeps=10),
         # the differentiable workload (131,072 particles on 64^3), a shorter rollout
         dict(name="rollout3d_131k", kind="rollout", dim=3, n=131_072, res=64, dtype="f32", substeps=20, checkpoint=10),
         # one corrected coarse step of the learned form at full size
@@ -592,7 +592,7 @@ def _exact_solver(c, seed):
 def _exact_batch2d(c, seed):
     scenes = _scenes(c, seed)
     out = [[], [], [], [], []]
-    if sum(len(s["x"]) for s in scenes) * c["substeps"] > 120_000_000:
+    if sum(len(s["x"]) for s in scenes) * c["substeps"] > 55_000_000:
         return None  # about 20 seconds
     for s in scenes:
         res, x0 = s["res"], s["x"]
