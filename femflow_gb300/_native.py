@@ -52,6 +52,7 @@ class Params(ctypes.Structure):
 
 
 MAX_PLANES = 8
+VARIANT_CELL_ORDER = 16  # ffmpm_params.variant bit 4
 PLANE_RULES = {"sticky": 0, "reference_literal": 1}
 
 

@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "mpm_kernels.cuh"
+#include "warp_kernels.cuh"
 
 namespace ffmpm {
 
@@ -57,6 +58,27 @@ bool valid_params(const ffmpm_params* p) {
     if (!(ss > 0.0)) return false;
   }
   return true;
+}
+
+// One substep (or one phase) on the caller's arrays without a block sort (warp_kernels.cuh): the
+// default outside the deterministic mode and the P2G variants.  Its grid pass reads every node, so a
+// grid that is large against the particle count keeps the sorted form, which visits the touched
+// blocks only.  Both sides at 4 to 17 M nodes: the dense pass costs 9 us at 2.1 M nodes and grows with
+// them (16 bytes a node), the sort and plan it saves 60 to 150 us.
+bool unsorted(const ffmpm_params& p, const Layout& L) {
+  return !p.deterministic && (p.variant & (kVariantP2GDirect | kVariantP2GLanes)) == 0 &&
+         L.nnodes <= std::max<int64_t>(int64_t(1) << 22, 16 * L.n);
+}
+
+// Whether such an operation's workspace has room for the counting sort by cell: float particles, and
+// more of them than are scattered as they come (kScatterMax).  Scattered in a random order a node
+// sums its particles one after another: at 30 particles a cell the float error of a substep's C was five
+// times that of sums over cells.  Up to 4096 particles that does not show (2,048 particles at 4 a cell:
+// the same error), and one launch does the work of four.
+constexpr int64_t kScatterMax = 4096;
+bool cell_sorted(const ffmpm_params& p, const Layout& L) {
+  return p.real_bytes == 4 && !p.deterministic && L.n > kScatterMax &&
+         L.nnodes <= std::max<int64_t>(int64_t(1) << 22, 16 * L.n);
 }
 
 }  // namespace
@@ -110,6 +132,14 @@ bool make_layout(const ffmpm_params& p, int64_t n, Layout* L) {
   // the plan kernels' per-block prefixes (3 x nblocks) and per-CTA totals and offsets
   L->off_plan_pref = take(sizeof(uint32_t) * 3 * L->nblocks);
   L->off_plan_cta = take(2 * 16 * ((L->nblocks + kPlanCta - 1) / kPlanCta));
+  // the counting sort by cell of the unsorted operations (warp_kernels.cuh): counters and first slots
+  // per node, and the records in cell order
+  if (cell_sorted(p, *L)) {
+    const size_t cells = align_up(size_t(L->nnodes), kCellTile);
+    L->off_cell_count = take(sizeof(uint32_t) * cells);
+    L->off_cell_start = take(sizeof(uint32_t) * cells);
+    L->off_recs = take(sizeof(float) * (p.dim == 3 ? RunRec<3>::kPacked : RunRec<2>::kPacked) * n);
+  }
   L->total = off;
   return true;
 }
@@ -179,6 +209,8 @@ struct Ws {
   void *gridA, *gridB, *stage;
   uint32_t* plan_pref;
   Scan4 *cta_tot, *cta_off;
+  uint32_t *cell_count, *cell_start;
+  void* recs;
 };
 
 Ws bind(void* ws, const Layout& L) {
@@ -204,6 +236,9 @@ Ws bind(void* ws, const Layout& L) {
   w.plan_pref = reinterpret_cast<uint32_t*>(w.base + L.off_plan_pref);
   w.cta_tot = reinterpret_cast<Scan4*>(w.base + L.off_plan_cta);
   w.cta_off = w.cta_tot + (L.nblocks + kPlanCta - 1) / kPlanCta;
+  w.cell_count = reinterpret_cast<uint32_t*>(w.base + L.off_cell_count);
+  w.cell_start = reinterpret_cast<uint32_t*>(w.base + L.off_cell_start);
+  w.recs = w.base + L.off_recs;
   return w;
 }
 
@@ -436,10 +471,80 @@ bool fused(const ffmpm_params& p, const Layout& L, int nsteps) {
          fused_smem_bytes(L) <= kMaxDynSmem;
 }
 
+// ---------------------------------------------------------------------------- unsorted operations
+// Launch shape of the warp kernels for `count` particles: whole CTAs while they fill the SMs, else
+// CTAs of 64 threads, so that a small count spreads over more SMs.
+template <typename T>
+struct WarpShape {
+  int threads, grid;
+  WarpShape(int64_t count, int per_sm) {
+    threads = kWarpCta<T>;
+    while (threads > 64 && (count + threads - 1) / threads < sm_count()) threads /= 2;
+    grid = work_grid((count + threads - 1) / threads, per_sm * (kWarpCta<T> / threads));
+  }
+};
+
+template <int DIM, typename T>
+void launch_p2g_warp(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, const uint32_t* perm,
+                     int64_t p0, int64_t p1, cudaStream_t s) {
+  const WarpShape<T> sh(p1 - p0, 8);
+  const size_t smem = sizeof(WarpRecs<DIM, T>) * (sh.threads / 32);
+  k_p2g_warp<DIM, T><<<sh.grid, sh.threads, smem, s>>>(kparams<T>(p), geom<DIM>(L), P, perm, (uint32_t)p0,
+                                                       (uint32_t)p1, static_cast<Node4<T>*>(w.gridA), &w.hdr->status,
+                                                       &w.hdr->polar_fallbacks);
+}
+
+// Scatter of the whole state into grid A.  Particles that may lie in any order are put in cell order
+// first; double particles, small counts and particles that the caller keeps in cell order
+// (kVariantCellOrder) are scattered as they come.
+template <int DIM, typename T>
+void scatter_unsorted(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, cudaStream_t s) {
+  if constexpr (sizeof(T) == 4) {
+    if (cell_sorted(p, L) && !(p.variant & kVariantCellOrder)) {
+      const KParams<T> kp = kparams<T>(p);
+      const uint32_t n = (uint32_t)L.n;
+      const unsigned pg = (n + kThreads - 1) / kThreads;
+      uint32_t* rank = w.keys0;
+      int* nodes = reinterpret_cast<int*>(w.vals0);
+      T* recs = static_cast<T*>(w.recs);
+      k_cell_rank<DIM, T><<<pg, kThreads, 0, s>>>(kp, L.R, P, n, w.cell_count, rank);
+      k_cell_offsets<<<(unsigned)((L.nnodes + kCellTile - 1) / kCellTile), kThreads, 0, s>>>(
+          w.cell_count, w.cell_start, w.hdr);
+      k_cell_records<DIM, T><<<pg, kThreads, 0, s>>>(kp, L.R, P, n, rank, w.cell_start, recs, nodes, &w.hdr->status,
+                                                     &w.hdr->polar_fallbacks);
+      const size_t smem = 2 * sizeof(WarpStage<DIM, T>);
+      k_cell_sums<DIM, T><<<(unsigned)((L.n + 191) / 192), 64, smem, s>>>(L.R, recs, nodes, w.hdr,
+                                                                          static_cast<Node4<T>*>(w.gridA));
+      return;
+    }
+  }
+  launch_p2g_warp<DIM, T>(p, L, w, P, nullptr, 0, L.n, s);
+}
+
+template <int DIM, typename T>
+void launch_grid_update_dense(const ffmpm_params& p, const Layout& L, const Ws& w, cudaStream_t s) {
+  k_grid_update_dense<DIM, T><<<work_grid((L.nnodes + 4 * kThreads - 1) / (4 * kThreads), 8), kThreads, 0, s>>>(
+      kparams<T>(p), geom<DIM>(L), w.hdr, static_cast<Node4<T>*>(w.gridA), static_cast<Node4<T>*>(w.gridB));
+}
+
+template <int DIM, typename T>
+void launch_g2p_range(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, int64_t p0, int64_t p1,
+                      cudaStream_t s) {
+  const WarpShape<T> sh(p1 - p0, 8);
+  k_g2p_range<DIM, T><<<sh.grid, sh.threads, 0, s>>>(kparams<T>(p), geom<DIM>(L), P, (uint32_t)p0, (uint32_t)p1,
+                                                     static_cast<const Node4<T>*>(w.gridB), &w.hdr->status);
+}
+
 // ------------------------------------------------------------------------------------ operations
 template <int DIM, typename T>
 int op_substep(const ffmpm_params& p, const Layout& L, const Ws& w, ffmpm_particles* P, cudaStream_t s) {
   const PView<T> pv = pview<T>(*P);
+  if (unsorted(p, L)) {
+    scatter_unsorted<DIM, T>(p, L, w, pv, s);
+    launch_grid_update_dense<DIM, T>(p, L, w, s);
+    launch_g2p_range<DIM, T>(p, L, w, pv, 0, L.n, s);
+    return check_launch();
+  }
   const uint32_t* perm = nullptr;
   sort_and_plan<DIM, T>(p, L, w, pv, false, &perm, s);
   if (p.deterministic) {
@@ -556,25 +661,19 @@ int op_substep_host(const ffmpm_params& p, const Layout& L, const Ws& w, const f
   const int64_t parts = int64_t(K) * (K + 1) / 2;
   auto up_lo = [&](int k) { return n * (int64_t(k) * (2 * K - k + 1) / 2) / parts; };
   auto lo = [&](int k) { return n * (int64_t(k) * (k + 1) / 2) / parts; };
-  const KParams<T> kp = kparams<T>(p);
-  const Geom<DIM> g = geom<DIM>(L);
   const PView<T> pv = pview<T>(*D);
-  const InternalSink<T> sink{static_cast<Node4<T>*>(w.gridA)};
   copy(false, 0, n, hp->up, true);
   for (int k = 0; k < K; ++k) {
     const int64_t a = up_lo(k), b = up_lo(k + 1);
     copy(false, a, b, hp->up);
     cudaEventRecord(hp->landed[k], hp->up);
     cudaStreamWaitEvent(s, hp->landed[k], 0);
-    k_p2g_range<DIM, T><<<work_grid((b - a + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
-        kp, g, pv, (uint32_t)a, (uint32_t)b, sink, &w.hdr->status, &w.hdr->polar_fallbacks);
+    launch_p2g_warp<DIM, T>(p, L, w, pv, nullptr, a, b, s);
   }
-  k_grid_update_dense<DIM, T><<<work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
-      kp, g, static_cast<Node4<T>*>(w.gridA), static_cast<Node4<T>*>(w.gridB));
+  launch_grid_update_dense<DIM, T>(p, L, w, s);
   for (int k = 0; k < K; ++k) {
     const int64_t a = lo(k), b = lo(k + 1);
-    k_g2p_range<DIM, T><<<work_grid((b - a + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
-        kp, g, pv, (uint32_t)a, (uint32_t)b, static_cast<const Node4<T>*>(w.gridB), &w.hdr->status);
+    launch_g2p_range<DIM, T>(p, L, w, pv, a, b, s);
     cudaEventRecord(hp->gathered[k], s);
     cudaStreamWaitEvent(hp->down, hp->gathered[k], 0);
     copy(true, a, b, hp->down);
@@ -703,6 +802,13 @@ template <int DIM, typename T>
 int op_p2g(const ffmpm_params& p, const Layout& L, const Ws& w, const ffmpm_particles* P, ffmpm_grid* grid,
            cudaStream_t s) {
   const PView<T> pv = pview<T>(*P);
+  if (unsorted(p, L)) {
+    scatter_unsorted<DIM, T>(p, L, w, pv, s);
+    k_grid_fold_user<DIM, T><<<work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
+        L.nnodes, w.hdr, static_cast<Node4<T>*>(w.gridA), static_cast<T*>(grid->velocity),
+        static_cast<T*>(grid->mass));
+    return check_launch();
+  }
   const uint32_t* perm = nullptr;
   sort_and_plan<DIM, T>(p, L, w, pv, false, &perm, s);
   if (p.deterministic) {
@@ -719,6 +825,12 @@ template <int DIM, typename T>
 int op_g2p(const ffmpm_params& p, const Layout& L, const Ws& w, const ffmpm_grid* grid, ffmpm_particles* P,
            cudaStream_t s) {
   const PView<T> pv = pview<T>(*P);
+  if (unsorted(p, L)) {
+    k_grid_pack_user<DIM, T><<<work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
+        L.nnodes, static_cast<const T*>(grid->velocity), w.hdr, static_cast<Node4<T>*>(w.gridB));
+    launch_g2p_range<DIM, T>(p, L, w, pv, 0, L.n, s);
+    return check_launch();
+  }
   const uint32_t* perm = nullptr;
   sort_and_plan<DIM, T>(p, L, w, pv, false, &perm, s);
   G2PExtra ex{};

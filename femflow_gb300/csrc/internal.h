@@ -24,7 +24,10 @@ struct WsHeader {
   uint32_t sort_now;   // sort cadence: 1 when this substep re-sorts (set by k_sort_decide)
   uint32_t far_stray;  // set by G2P when a particle left the neighbourhood its block's plan covers
   uint32_t det_next[2];  // deterministic P2G: next entry of the occupied list, per pass (zeroed per launch)
-  uint32_t pad[54];
+  uint32_t b_dirty;  // the velocity grid has held a non-finite value (see k_grid_update_dense)
+  uint32_t cell_cursor;  // slots handed out by k_cell_offsets (zeroed by the grid pass that follows)
+  uint32_t cell_occupied;  // cells with particles, as counted by k_cell_offsets (zeroed with it)
+  uint32_t pad[51];
 };
 static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
 
@@ -35,7 +38,7 @@ struct Layout {
   int64_t n = 0, nblocks = 0, nnodes = 0, max_chunks = 0, ntiles = 0;
   size_t off_block_count = 0, off_block_start = 0, off_block_cnt = 0, off_chunks = 0, off_touched = 0, off_tmark = 0,
          off_occupied = 0, off_keys_next = 0, off_keys0 = 0, off_keys1 = 0, off_vals0 = 0, off_vals1 = 0,
-         off_hist = 0, off_gridA = 0, off_gridB = 0, off_stage = 0, off_plan_pref = 0, off_plan_cta = 0, total = 0;
+         off_hist = 0, off_gridA = 0, off_gridB = 0, off_stage = 0, off_plan_pref = 0, off_plan_cta = 0, off_cell_count = 0, off_cell_start = 0, off_recs = 0, total = 0;
 };
 
 bool make_layout(const ffmpm_params& p, int64_t n, Layout* L);

@@ -22,7 +22,7 @@ Gradients with respect to Young's modulus and Poisson's ratio follow by autograd
 from __future__ import annotations
 
 import ctypes
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 
 import torch
 
@@ -45,6 +45,8 @@ class RolloutConfig:
     # planar colliders ((point, normal) pairs) applied by every grid update, and their rule
     planes: tuple = ()
     plane_rule: str = "sticky"
+    # the particles come in (about) the order of their base cells: ``simulate`` sets it when it orders them
+    cell_order: bool = False
 
 
 def lame(E_mod, nu):
@@ -85,7 +87,8 @@ class _Runner:
         self.device = device
         self.params = E.make_params(dim, cfg.res, dtype, 1.0 / cfg.res, float(cfg.res), cfg.dt, cfg.gravity,
                                     cfg.volume, cfg.hardening, model=cfg.model, wall_mode=cfg.wall_mode,
-                                    planes=cfg.planes, plane_rule=cfg.plane_rule)
+                                    planes=cfg.planes, plane_rule=cfg.plane_rule,
+                                    variant=N.VARIANT_CELL_ORDER if cfg.cell_order else 0)
         if torch.is_tensor(mass):
             self.mass = mass.detach().to(device=device, dtype=dtype).reshape(n).contiguous()
         else:
@@ -223,5 +226,6 @@ def simulate(x0, v0, mu_0, lambda_0, cfg: RolloutConfig, mass, F0=None, C0=None,
     inv = torch.empty_like(perm)
     inv[perm] = torch.arange(n, device=perm.device)
     pick = lambda t: t[perm] if torch.is_tensor(t) and t.dim() >= 1 and t.shape[0] == n else t
+    cfg = replace(cfg, cell_order=True)
     out = MPMRollout.apply(pick(x0), pick(v0), pick(F0), pick(C0), pick(mu), pick(lam), pick(mass), cfg)
     return tuple(o[inv] for o in out)
