@@ -354,20 +354,13 @@ size_t tile_smem(const Layout& L) {
 // Dynamic shared memory every kernel may use (set_smem raises each kernel's limit to it).
 constexpr size_t kMaxDynSmem = 200 * 1024;
 
-// Dynamic shared memory of the cell-run P2G and of the fused G2P + P2G for this layout.
+// Dynamic shared memory of the cell-run P2G for this layout.
 size_t cells_smem_bytes(const Layout& L) {
   if (L.real_bytes == 4)
     return L.dim == 3 ? tile_smem<3, float>(L) + cell_run_smem_bytes<3, float>(L.bs)
                       : tile_smem<2, float>(L) + cell_run_smem_bytes<2, float>(L.bs);
   return L.dim == 3 ? tile_smem<3, double>(L) + cell_run_smem_bytes<3, double>(L.bs)
                     : tile_smem<2, double>(L) + cell_run_smem_bytes<2, double>(L.bs);
-}
-
-size_t fused_smem_bytes(const Layout& L) {
-  const int tn = L.dim == 3 ? L.tile * L.tile * L.tile : L.tile * L.tile;
-  if (L.real_bytes == 4)
-    return L.dim == 3 ? g2p2g_smem_bytes<3, float>(tn, L.bs) : g2p2g_smem_bytes<2, float>(tn, L.bs);
-  return L.dim == 3 ? g2p2g_smem_bytes<3, double>(tn, L.bs) : g2p2g_smem_bytes<2, double>(tn, L.bs);
 }
 
 // Raise a kernel's dynamic shared-memory limit once per kernel (a host-side attribute call,
@@ -446,29 +439,11 @@ int launch_g2p(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<
   return FFMPM_OK;
 }
 
-template <int DIM, typename T>
-int launch_g2p2g(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& Pin, const PView<T>& Pout,
-                 const uint32_t* perm, const G2PExtra& ex, cudaStream_t s, const uint32_t* flag) {
-  alignas(64) CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  if (!encode_grid_map(&map, w.gridB, L)) return FFMPM_ERR_CUDA;
-  const int tn = DIM == 3 ? L.tile * L.tile * L.tile : L.tile * L.tile;
-  const size_t smem = g2p2g_smem_bytes<DIM, T>(tn, L.bs);
-  auto kern = k_g2p2g<DIM, T>;
-  set_smem(kern, smem);
-  kern<<<work_grid(L.max_chunks, resident_per_sm(kern, smem)), kThreads, smem, s>>>(
-      kparams<T>(p), geom<DIM>(L), Pin, Pout, perm, w.chunks, w.hdr, map, ex,
-      InternalSink<T>{static_cast<Node4<T>*>(w.gridA)}, w.tmark, w.touched, &w.hdr->status, &w.hdr->polar_fallbacks,
-      flag);
-  return FFMPM_OK;
-}
-
 // Fused G2P + P2G in the sorted solver: the default outside the deterministic mode and the P2G
-// variants, for runs of two or more substeps whose two tiles and records fit in shared memory.
+// variants, for runs of two or more substeps (3D blocks of 16 nodes a side keep separate launches).
 bool fused(const ffmpm_params& p, const Layout& L, int nsteps) {
   return !p.deterministic && nsteps >= 2 &&
-         (p.variant & (kVariantNoFuse | kVariantP2GDirect | kVariantP2GLanes)) == 0 &&
-         fused_smem_bytes(L) <= kMaxDynSmem;
+         (p.variant & (kVariantNoFuse | kVariantP2GDirect | kVariantP2GLanes)) == 0 && !(L.dim == 3 && L.bs > 8);
 }
 
 // ---------------------------------------------------------------------------- unsorted operations
@@ -492,6 +467,17 @@ void launch_p2g_warp(const ffmpm_params& p, const Layout& L, const Ws& w, const 
   k_p2g_warp<DIM, T><<<sh.grid, sh.threads, smem, s>>>(kparams<T>(p), geom<DIM>(L), P, perm, (uint32_t)p0,
                                                        (uint32_t)p1, static_cast<Node4<T>*>(w.gridA), &w.hdr->status,
                                                        &w.hdr->polar_fallbacks);
+}
+
+// G2P of a sorted run, with the next substep's P2G (kNext) or alone.
+template <int DIM, typename T, bool kNext>
+void launch_g2p_sorted(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& Pin, const PView<T>& Pout,
+                       const uint32_t* perm, const G2PExtra& ex, cudaStream_t s) {
+  const WarpShape<T> sh(L.n, 8);
+  const size_t smem = kNext ? sizeof(WarpRecs<DIM, T>) * (sh.threads / 32) : 0;
+  k_g2p_sorted<DIM, T, kNext><<<sh.grid, sh.threads, smem, s>>>(kparams<T>(p), geom<DIM>(L), Pin, Pout, perm,
+                                                                 (uint32_t)L.n, ex, static_cast<Node4<T>*>(w.gridA),
+                                                                 w.hdr, w.tmark, w.touched);
 }
 
 // Scatter of the whole state into grid A.  Particles that may lie in any order are put in cell order
@@ -722,7 +708,7 @@ int op_substeps_fused(const ffmpm_params& p, const Layout& L, const Ws& w, PView
   sort_and_plan<DIM, T>(p, L, w, va, false, &sorted_perm, s, tm, nullptr, 1);
   const uint32_t* perm = sorted_perm;  // the permutation the next P2G / G2P applies (null: none)
   if (tm) tm->begin(3);
-  launch_p2g<DIM, T>(p, L, w, va, perm, InternalSink<T>{static_cast<Node4<T>*>(w.gridA)}, s);
+  launch_p2g_warp<DIM, T>(p, L, w, va, perm, 0, L.n, s);
   if (tm) tm->end(1);
   for (int k = 0; k < nsteps; ++k) {
     const PView<T>& in = (k & 1) ? vb : va;
@@ -736,9 +722,8 @@ int op_substeps_fused(const ffmpm_params& p, const Layout& L, const Ws& w, PView
       // k >= 1: the buffer is already in the order of the current plan
       G2PExtra ex{ids_in, ids_out, nullptr, nullptr, L.cell_bits, w.gridB, nullptr};
       if (tm) tm->begin(5);
-      const int rc = launch_g2p<DIM, T, true, true>(p, L, w, in, out, nullptr, nullptr, ex, s);
+      launch_g2p_sorted<DIM, T, false>(p, L, w, in, out, nullptr, ex, s);
       if (tm) tm->end(1);
-      if (rc != FFMPM_OK) return rc;
       snapshot<DIM, T>(snap, k, out, ids_out, L.n, s);
       break;
     }
@@ -748,9 +733,8 @@ int op_substeps_fused(const ffmpm_params& p, const Layout& L, const Ws& w, PView
     G2PExtra ex{ids_in, ids_out, keys ? w.keys_next : nullptr, keys ? w.block_count : nullptr, L.cell_bits, w.gridB,
                 nullptr};
     if (tm) tm->begin(6);
-    const int rc = launch_g2p2g<DIM, T>(p, L, w, in, out, perm, ex, s, nullptr);
+    launch_g2p_sorted<DIM, T, true>(p, L, w, in, out, perm, ex, s);
     if (tm) tm->end(1);
-    if (rc != FFMPM_OK) return rc;
     snapshot<DIM, T>(snap, k, out, ids_out, L.n, s);
   }
   return check_launch();

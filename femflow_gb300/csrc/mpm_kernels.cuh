@@ -10,7 +10,6 @@
 //                  blocks only                               (three_d/grid_op.py:5-67)
 //   k_g2p          TMA-staged tile of grid velocities, gather v and APIC C, advect, update F
 //                                                            (three_d/g2p.py:9-59)
-//   k_g2p2g        G2P of one substep fused with P2G of the next (resident solver)
 // Sorting and planning run on the substeps that re-sort; the others keep the plan.
 #pragma once
 
@@ -281,7 +280,9 @@ __device__ __forceinline__ void block_exclusive_scan4_parts(const Scan4 (&v)[KB]
 }
 
 // Touched test of block b, gather form: any block b - o, o in {0,1}^DIM, holds particles; with `sym`
-// any block b + o, o in {-1,0,1}^DIM (the histogram is small and stays in L2).
+// any block b + o, o in {-1,0,1}^DIM (the histogram is small and stays in L2).  With `sym` the mark is 2
+// where an occupied block lies at b + o, o in {0,1}^DIM: the blocks b + {0,1}^DIM, which the stencils based
+// in b reach, are then touched too.
 template <int DIM>
 __device__ __forceinline__ uint32_t plan_touched(const Geom<DIM>& g, const uint32_t* __restrict__ block_count, int b,
                                                  int sym) {
@@ -303,13 +304,15 @@ __device__ __forceinline__ uint32_t plan_touched(const Geom<DIM>& g, const uint3
     return 0u;
   }
   constexpr int NO = DIM == 3 ? 27 : 9;
+  uint32_t mark = 0u;
 #pragma unroll
   for (int o = 0; o < NO; ++o) {
     int nb_id = 0, r = o;
-    bool ok = true;
+    bool ok = true, above = true;
 #pragma unroll
     for (int d = DIM - 1; d >= 0; --d) {
       const int cc = bc[d] + (r % 3) - 1;
+      above = above && r % 3 > 0;
       r /= 3;
       ok = ok && cc >= 0 && cc < g.nb;
     }
@@ -322,9 +325,9 @@ __device__ __forceinline__ uint32_t plan_touched(const Geom<DIM>& g, const uint3
       mul *= g.nb;
       r /= 3;
     }
-    if (block_count[nb_id] > 0) return 1u;
+    if (block_count[nb_id] > 0) mark = above ? 2u : max(mark, 1u);
   }
-  return 0u;
+  return mark;
 }
 
 constexpr int kPlanCta = 1024;  // blocks per CTA of the plan kernels
@@ -346,7 +349,7 @@ __global__ void __launch_bounds__(kPlanCta) k_plan_local(Geom<DIM> g, const uint
     c = block_count[b];
     tch = plan_touched<DIM>(g, block_count, b, sym);
   }
-  const Scan4 v[1] = {Scan4{c, (c + kChunk - 1) / kChunk, tch, c > 0 ? 1u : 0u}};
+  const Scan4 v[1] = {Scan4{c, (c + kChunk - 1) / kChunk, tch > 0 ? 1u : 0u, c > 0 ? 1u : 0u}};
   Scan4 ex[1], tot;
   block_exclusive_scan4_parts<1>(v, ex, &tot, part_buf);
   if (b < g.nblocks) {
@@ -1990,158 +1993,6 @@ __global__ void __launch_bounds__(kThreads) k_g2p(KParams<T> kp, Geom<DIM> g, PV
       g2p_particle<DIM, T>(kp, g, Pin, Pout, p1, kSorted ? s1 : p1, org, tile, status, kSorted, ex, in1);
       if (two) g2p_particle<DIM, T>(kp, g, Pin, Pout, p2, kSorted ? s2 : p2, org, tile, status, kSorted, ex, in2);
     }
-  }
-}
-
-// ----------------------------------------------------------------------------------------------
-// Fused G2P + P2G: substep k's G2P and substep k+1's P2G in one pass over the particles.  The
-// updated particle (x, v, C, F) goes straight from the gather into the next substep's record, so
-// v and C never travel through memory between the two, and x and F are read once per substep.
-// Both halves use the chunk's block: the G2P tile of grid velocities (staged by TMA from the
-// workspace's velocity grid) and the P2G tile of momentum/mass (flushed into the workspace's
-// accumulation grid), and the cell-run phases of k_p2g_cells.  The block plan was made from the
-// positions of substep k, so a particle's new stencil may leave its block's tile (it takes the
-// direct global adds) or, moving fast, the blocks the plan touches: it then adds the blocks its
-// stencil covers to the touched list itself, so that the grid update visits every node that
-// received mass.
-
-// Add the blocks covered by the stencil at `base` to the touched list (each block once: `tmark`
-// holds 1 for every listed block).
-template <int DIM>
-__device__ __forceinline__ void mark_touched(const Geom<DIM>& g, const int base[DIM], uint32_t* tmark,
-                                             uint32_t* touched, uint32_t* n_touched) {
-  int lo[DIM], ext[DIM];
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) {
-    lo[d] = base[d] >> g.bs_shift;
-    ext[d] = min((base[d] + 2) >> g.bs_shift, g.nb - 1) - lo[d];  // 0 or 1
-  }
-  for (int o = 0; o < (1 << DIM); ++o) {
-    int id = 0;
-    bool ok = true;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      const int od = (o >> (DIM - 1 - d)) & 1;
-      ok = ok && od <= ext[d];
-      id = id * g.nb + lo[d] + od;
-    }
-    if (ok && atomicCAS(&tmark[id], 0u, 1u) == 0u) touched[atomicAdd(n_touched, 1u)] = (uint32_t)id;
-  }
-}
-
-// Dynamic shared memory of k_g2p2g: [pad to 128 B][G2P tile: TN Node4][mbarrier: 128 B]
-// [P2G tile: 4 TN reals][cell-run arrays], every region starting on 128 bytes.
-__host__ __device__ constexpr size_t align128(size_t v) { return (v + 127) & ~size_t(127); }
-
-template <int DIM, typename T>
-__host__ __device__ constexpr size_t g2p2g_smem_bytes(int TN, int bs) {
-  return 128 + align128(size_t(TN) * sizeof(Node4<T>)) + 128 + align128(size_t(4) * TN * sizeof(T)) +
-         cell_run_smem_bytes<DIM, T>(bs);
-}
-
-template <int DIM, typename T>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_g2p2g(
-    KParams<T> kp, Geom<DIM> g, PView<T> Pin, PView<T> Pout, const uint32_t* __restrict__ perm,
-    const int4* __restrict__ chunks, WsHeader* hdr, const __grid_constant__ CUtensorMap tmap, G2PExtra ex,
-    InternalSink<T> sink, uint32_t* __restrict__ tmark, uint32_t* __restrict__ touched, int32_t* status,
-    uint32_t* fallbacks, const uint32_t* __restrict__ sort_flag) {
-  if (sort_flag && *sort_flag == 0u) perm = nullptr;  // plan kept from an earlier substep: identity order
-  if (perm && wait_gave_up(status)) return;
-  constexpr int RS = RecLayout<DIM>::kStride;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int TN = tile_nodes<DIM>(g);
-  unsigned char* at = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-  Node4<T>* gtile = reinterpret_cast<Node4<T>*>(at);
-  at += align128(size_t(TN) * sizeof(Node4<T>));
-  uint64_t& bar = *reinterpret_cast<uint64_t*>(at);
-  at += 128;
-  T* ptile = reinterpret_cast<T*>(at);
-  at += align128(size_t(4) * TN * sizeof(T));
-  __shared__ int nruns_s;
-  __shared__ int warp_cnt[kThreads / 32];
-  __shared__ int warp_nz[kThreads / 32];
-  const CellRunSmem<T> cr = cell_run_smem<DIM, T>(at, g, &nruns_s, warp_cnt, warp_nz);
-  const TileAdder<DIM, T> tacc{ptile, TN, g.tile};
-  const uint32_t nch = hdr->n_chunks;
-  const uint32_t per = (nch + gridDim.x - 1) / gridDim.x;
-  const uint32_t c0 = blockIdx.x * per;
-  const uint32_t c1 = min(nch, c0 + per);
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    fence_barrier_init();
-  }
-  __syncthreads();
-  uint32_t phase = 0;
-  int cur = -1;
-  int org[DIM];
-  for (uint32_t c = c0; c < c1; ++c) {
-    const int4 ch = chunks[c];
-    if (ch.x != cur) {
-      if (cur >= 0) {
-        __syncthreads();  // phase 3 of the previous chunk is done with the P2G tile
-        p2g_flush<DIM, T, InternalSink<T>>(ptile, TN, g, org, sink);
-      }
-      __syncthreads();  // every thread is done with both tiles
-      cur = ch.x;
-      int bc[DIM];
-      block_coords<DIM>(g, cur, bc);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) org[d] = bc[d] * g.bs;
-      if (threadIdx.x == 0) {
-        mbar_arrive_expect_tx(&bar, (uint32_t)(TN * sizeof(Node4<T>)));
-        if constexpr (DIM == 3)
-          tma_load_4d(gtile, &tmap, &bar, 0, org[2], org[1], org[0]);
-        else
-          tma_load_3d(gtile, &tmap, &bar, 0, org[1], org[0]);
-      }
-      for (int t = threadIdx.x; t < 4 * TN; t += blockDim.x) ptile[t] = T(0);
-      const bool timed_out = !mbar_wait(&bar, phase);
-      if (__syncthreads_or(timed_out)) {
-        // the tile copy may still be in flight: wait for it once more (bounded) so that it does not
-        // land in shared memory after this CTA has left
-        if (threadIdx.x == 0) {
-          raise_status(status, FFMPM_STATUS_TIMEOUT);
-          mbar_wait(&bar, phase);
-        }
-        __syncthreads();
-        return;
-      }
-      phase ^= 1u;
-    }
-    // phase 1: G2P of substep k, then the record of substep k+1, one particle per thread
-    for (int l = threadIdx.x; l < ch.z; l += blockDim.x) {
-      const uint32_t s = ch.y + l;
-      const uint32_t p = perm ? perm[s] : s;
-      G2PIn<DIM, T> in;
-      g2p_load<DIM, T>(Pin, p, true, in);
-      P2GIn<DIM, T> nx;
-      T rec[RS];
-      int cell = -1, base[DIM];
-      int kind = kRecOut;
-      if (g2p_particle<DIM, T, true>(kp, g, Pin, Pout, p, s, org, gtile, status, true, ex, in, &nx)) {
-        kind = p2g_record<DIM, T>(kp, g, nx, org, rec, cell, status, fallbacks, base);
-        if (kind == kRecStray) {
-          // outside the blocks within +-1 of the chunk's block (which the plan always touches)
-          bool far = false;
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            const int lb = base[d] - org[d];
-            far = far || lb < -g.bs || lb > 2 * g.bs - 3;
-          }
-          if (far) mark_touched<DIM>(g, base, tmark, touched, &hdr->n_touched);
-        }
-      }
-      p2g_store_record<DIM, T>(cr, l, rec, kind, cell, base);
-    }
-    __syncthreads();
-    for (int l = threadIdx.x; l < ch.z; l += blockDim.x)
-      if (cr.cells[l] == -2) p2g_scatter_record<DIM, T, InternalSink<T>>(cr.recs + (size_t)l * RS, g.R, sink);
-    p2g_cell_runs<DIM, T>(cr, g, ch.z, tacc);
-    __syncthreads();  // records and runs are rewritten by the next chunk
-  }
-  if (cur >= 0) {
-    __syncthreads();
-    p2g_flush<DIM, T, InternalSink<T>>(ptile, TN, g, org, sink);
   }
 }
 

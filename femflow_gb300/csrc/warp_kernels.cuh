@@ -24,10 +24,10 @@ struct RunRec {
 
 template <int DIM, typename T>
 __device__ __forceinline__ int run_record(const KParams<T>& kp, const P2GIn<DIM, T>& in, int R,
-                                          T (&rec)[RunRec<DIM>::kPacked], int32_t* status, uint32_t* fallbacks) {
+                                          T (&rec)[RunRec<DIM>::kPacked], int32_t* status, uint32_t* fallbacks,
+                                          int (&base)[DIM]) {
   constexpr int DD = DIM * DIM, a0 = 1 + DIM;
   T fx[DIM];
-  int base[DIM];
   bool ok = true;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) ok = ok && base_of(in.x[d], kp.inv_dx, kp.res, base[d], fx[d]);
@@ -302,7 +302,8 @@ __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom
     if (s + lane < p1) {
       P2GIn<DIM, T> in;
       p2g_load<DIM, T>(kp, P, perm ? perm[s + lane] : s + lane, in);
-      node = run_record<DIM, T>(kp, in, g.R, rec, status, fallbacks);
+      int base[DIM];
+      node = run_record<DIM, T>(kp, in, g.R, rec, status, fallbacks, base);
     }
     warp_scatter<DIM, T>(wr, rec, node, ln, A, g.R);
   }
@@ -415,7 +416,8 @@ __global__ void __launch_bounds__(kThreads) k_cell_records(KParams<T> kp, int R,
   p2g_load<DIM, T>(kp, P, p, in);
   const uint32_t rk = rank[p];
   T rec[RunRec<DIM>::kPacked];
-  const int node = run_record<DIM, T>(kp, in, R, rec, status, fallbacks);
+  int base[DIM];
+  const int node = run_record<DIM, T>(kp, in, R, rec, status, fallbacks, base);
   if (node < 0) return;
   const uint32_t at = start[node] + rk;
   nodes[at] = node;
@@ -568,6 +570,83 @@ __global__ void __launch_bounds__(kWarpCta<T>) k_g2p_range(KParams<T> kp, Geom<D
     G2PIn<DIM, T> in;
     g2p_load<DIM, T>(P, p, need_jp, in);
     g2p_particle<DIM, T>(kp, g, P, P, p, p, org, nullptr, status, false, ex, in);
+  }
+}
+
+// ----------------------------------------------------------------------------------------------
+// Fused G2P + P2G of the resident solver: substep k's G2P and substep k+1's P2G in one pass over the
+// particles.  The updated particle (x, v, C, F) goes straight from the gather into the next substep's
+// record, so v and C never travel through memory between the two, and x and F are read once per
+// substep.  A warp takes 32 particles of the solver's cell order: its gathers fall on the nodes of a few
+// cells, its scatter is warp_scatter's (the particles that crossed a cell boundary since the last re-sort
+// join the run of their new cell there).  The grid update visits the blocks the plan touches: a
+// particle whose new stencil may leave them adds the blocks it covers to the list itself.
+// Two cubes of 1,048,576 particles on 128^3 (GB300): 122 us a launch; chunks of 512 particles with a
+// shared-memory tile for each side, an in-chunk counting sort and CTA barriers between the phases took
+// 156.  16,384 particles on 64^3: 13 us a substep against 38 (512 one-warp batches instead of 32 chunks).
+// Bound by instruction issue and the latency of the gathers.
+
+// Add the blocks covered by the stencil at `base` to the touched list (each block once: `tmark` is
+// nonzero for every listed block; 2 where the blocks of every stencil based in the block are listed).
+template <int DIM>
+__device__ __forceinline__ void mark_touched(const Geom<DIM>& g, const int base[DIM], uint32_t* tmark,
+                                             uint32_t* touched, uint32_t* n_touched) {
+  int lo[DIM], ext[DIM];
+  int id = 0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    lo[d] = base[d] >> g.bs_shift;
+    ext[d] = min((base[d] + 2) >> g.bs_shift, g.nb - 1) - lo[d];  // 0 or 1
+    id = id * g.nb + lo[d];
+  }
+  if (__ldcg(&tmark[id]) == 2u) return;
+  for (int o = 0; o < (1 << DIM); ++o) {
+    int at = 0;
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const int od = (o >> (DIM - 1 - d)) & 1;
+      ok = ok && od <= ext[d];
+      at = at * g.nb + lo[d] + od;
+    }
+    if (ok && __ldcg(&tmark[at]) == 0u && atomicCAS(&tmark[at], 0u, 1u) == 0u)
+      touched[atomicAdd(n_touched, 1u)] = (uint32_t)at;
+  }
+}
+
+// kNext: G2P and the next substep's P2G; else the last substep's G2P alone (which writes v and C).
+template <int DIM, typename T, bool kNext>
+__global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 2 : 1) k_g2p_sorted(
+    KParams<T> kp, Geom<DIM> g, PView<T> Pin, PView<T> Pout, const uint32_t* __restrict__ perm, uint32_t n,
+    G2PExtra ex, Node4<T>* __restrict__ A, WsHeader* hdr, uint32_t* __restrict__ tmark,
+    uint32_t* __restrict__ touched) {
+  int32_t* const status = &hdr->status;
+  if (perm && wait_gave_up(status)) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  WarpRecs<DIM, T>& wr = reinterpret_cast<WarpRecs<DIM, T>*>(smem_raw)[kNext ? threadIdx.x >> 5 : 0];
+  const RunLane<DIM, T> ln;
+  const int lane = threadIdx.x & 31;
+  int org[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) org[d] = -(1 << 24);  // no staged tile: every stencil is off-tile
+  for (uint32_t s0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); s0 < n; s0 += gridDim.x * blockDim.x) {
+    const uint32_t s = s0 + lane;
+    T rec[RunRec<DIM>::kPacked];
+    int node = -1;
+    if (s < n) {
+      const uint32_t p = perm ? perm[s] : s;
+      G2PIn<DIM, T> in;
+      g2p_load<DIM, T>(Pin, p, true, in);
+      P2GIn<DIM, T> nx;
+      if (g2p_particle<DIM, T, kNext>(kp, g, Pin, Pout, p, s, org, nullptr, status, true, ex, in, &nx)) {
+        if constexpr (kNext) {
+          int base[DIM];
+          node = run_record<DIM, T>(kp, nx, g.R, rec, status, &hdr->polar_fallbacks, base);
+          if (node >= 0) mark_touched<DIM>(g, base, tmark, touched, &hdr->n_touched);
+        }
+      }
+    }
+    if constexpr (kNext) warp_scatter<DIM, T>(wr, rec, node, ln, A, g.R);
   }
 }
 
