@@ -4,8 +4,8 @@
 // Phases, separated by a grid-wide barrier (bounded spin; co-residency of all CTAs is guaranteed by
 // the cooperative launch):
 //   P2G over every particle of every scene: stress (utils.py:52-92) + 9-node scatter into the
-//     scene's grid A (two_d/p2g.py:11-76); the lanes of a warp that share a base cell sum their
-//     contributions before the atomics, and every scene's box of touched nodes is widened
+//     scene's grid A (two_d/p2g.py:11-76) by warp_scatter (warp_kernels.cuh): particles that share a
+//     base cell are summed before the atomics; every scene's box of touched nodes is widened
 //   then per substep:
 //   grid update over the nodes of every scene's box: two_d/grid_op.py:5-24 into B, A re-zeroed
 //   G2P over every particle (gather v and C from B, advect, F update, Jp: two_d/g2p.py:5-47),
@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "mpm_kernels.cuh"
+#include "warp_kernels.cuh"
 
 namespace ffmpm {
 namespace {
@@ -206,81 +207,40 @@ __device__ __forceinline__ void widen_box(int* bx, int lo0, int lo1, int hi0, in
   if (hi1 > __ldcg(bx + 3)) atomicMax(bx + 3, hi1);
 }
 
-// P2G of one particle per lane of a whole warp (every lane calls it).  Lanes that hold a run of
-// consecutive particles with the same base node (the batch keeps each scene's particles ordered by
-// base cell) sum their 27 node contributions with shuffles; the run's first lane then adds the 9
-// sums to the grid, one vector atomic per node instead of one per (particle, node).  The scene's
-// box of touched nodes is widened by one atomic per bound per warp where the warp holds one scene.
+// P2G of one particle per lane of a whole warp (every lane calls it) through warp_scatter, the lanes of
+// one scene at a time (a warp nearly always holds one).  256 scenes of 4.4M particles, 10 substeps a call
+// (GB300): 3,266 us, from 4,050 with the nodes' contributions summed by shuffles over runs of lanes;
+// bound by instruction issue.  32 warps per SM pay more than the registers they take away: 4,310 us with
+// 16.  Shares of neighbouring particles per warp, instead of the launch-wide stride, take 4,250: every
+// warp then streams rows of its own.  The box of touched nodes of each scene is widened
+// by one atomic per bound per warp.
 template <typename T>
-__device__ __forceinline__ void scatter_warp(Node4<T>* A, int64_t noff, int* boxes, int si, bool ok, const int b[2],
-                                             const T fx[2], const T v[2], const T A2[4], const KParams<T>& kp,
-                                             int lane) {
+__device__ __forceinline__ void scatter_warp(WarpRecs<2, T>& wr, const RunLane<2, T>& ln, Node4<T>* A,
+                                             const int64_t* noff, int* boxes, int si, bool ok, const int b[2],
+                                             const T fx[2], const T v[2], const T A2[4], const KParams<T>& kp) {
   constexpr unsigned kFull = 0xffffffffu;
-  T w[3][2];
-#pragma unroll
-  for (int d = 0; d < 2; ++d) {
-    T ww[3];
-    bspline(ok ? fx[d] : T(0), ww);
-    w[0][d] = ww[0];
-    w[1][d] = ww[1];
-    w[2][d] = ww[2];
-  }
+  const int lane = threadIdx.x & 31;
   const int R = kp.res + 1;
-  // runs: a lane starts one when its base node differs from the previous lane's (or it holds no
-  // particle); lanes of one run carry the same run number
-  const int64_t key = ok ? noff + (int64_t)b[0] * R + b[1] : -1 - (int64_t)lane;
-  const int64_t prev = __shfl_up_sync(kFull, key, 1);
-  const bool head = lane == 0 || key != prev;
-  const unsigned heads = __ballot_sync(kFull, head);
-  const int run = __popc(heads & (kFull >> (31 - lane)));  // heads at or below this lane
-  const bool shared = heads != kFull;                         // some run holds more than one particle
-  bool same[5];
+  T rec[RunRec<2>::kPacked];
+  rec[0] = kp.mass;
+  rec[1] = v[0] * kp.mass - kp.dx * (A2[0] * fx[0] + A2[1] * fx[1]);
+  rec[2] = v[1] * kp.mass - kp.dx * (A2[2] * fx[0] + A2[3] * fx[1]);
 #pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const int off = 1 << s;
-    const int other = __shfl_down_sync(kFull, run, off);
-    same[s] = lane + off < 32 && other == run;
-  }
-  Node4<T>* grid = A + noff;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const T d0 = (T(i) - fx[0]) * kp.dx;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const T d1 = (T(j) - fx[1]) * kp.dx;
-      const T wt = w[i][0] * w[j][1];
-      T qx = ok ? wt * (v[0] * kp.mass + (A2[0] * d0 + A2[1] * d1)) : T(0);
-      T qy = ok ? wt * (v[1] * kp.mass + (A2[2] * d0 + A2[3] * d1)) : T(0);
-      T qm = ok ? wt * kp.mass : T(0);
-      if (shared) {
-        // suffix sums within each run: after the five steps the run's first lane holds its total
-#pragma unroll
-        for (int s = 0; s < 5; ++s) {
-          const int off = 1 << s;
-          const T tx = __shfl_down_sync(kFull, qx, off);
-          const T ty = __shfl_down_sync(kFull, qy, off);
-          const T tm = __shfl_down_sync(kFull, qm, off);
-          if (same[s]) {
-            qx += tx;
-            qy += ty;
-            qm += tm;
-          }
-        }
-      }
-      if (ok && head) InternalSink<T>{grid}.add((int64_t)(b[0] + i) * R + (b[1] + j), qx, qy, T(0), qm);
-    }
-  }
-  int lo0 = ok ? b[0] : kEmptyLo, lo1 = ok ? b[1] : kEmptyLo;
-  int hi0 = ok ? b[0] + 2 : kEmptyHi, hi1 = ok ? b[1] + 2 : kEmptyHi;
-  const int si0 = __shfl_sync(kFull, si, 0);
-  if (__all_sync(kFull, !ok || si == si0)) {
-    lo0 = __reduce_min_sync(kFull, lo0);
-    lo1 = __reduce_min_sync(kFull, lo1);
-    hi0 = __reduce_max_sync(kFull, hi0);
-    hi1 = __reduce_max_sync(kFull, hi1);
-    if (lane == 0 && lo0 != kEmptyLo) widen_box(boxes + 4 * si0, lo0, lo1, hi0, hi1);
-  } else if (ok) {
-    widen_box(boxes + 4 * si, lo0, lo1, hi0, hi1);
+  for (int i = 0; i < 4; ++i) rec[3 + i] = kp.dx * A2[i];
+  rec[7] = fx[0];
+  rec[8] = fx[1];
+  rec[9] = rec[10] = rec[11] = T(0);
+  for (unsigned left = __ballot_sync(kFull, ok); left;) {
+    const int lead = __ffs(left) - 1;
+    const int s = __shfl_sync(kFull, si, lead), Rs = __shfl_sync(kFull, R, lead);
+    const bool mine = ok && si == s;
+    warp_scatter<2, T>(wr, rec, mine ? b[0] * R + b[1] : -1, ln, A + noff[s], Rs);
+    const int lo0 = __reduce_min_sync(kFull, mine ? b[0] : kEmptyLo);
+    const int lo1 = __reduce_min_sync(kFull, mine ? b[1] : kEmptyLo);
+    const int hi0 = __reduce_max_sync(kFull, mine ? b[0] + 2 : kEmptyHi);
+    const int hi1 = __reduce_max_sync(kFull, mine ? b[1] + 2 : kEmptyHi);
+    if (lane == 0) widen_box(boxes + 4 * s, lo0, lo1, hi0, hi1);
+    left &= ~__ballot_sync(kFull, mine);
   }
 }
 
@@ -320,7 +280,7 @@ __device__ __forceinline__ void load_boxes(const int* box, const SceneK<T>* s_sc
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned char* ws, PView<T> P, int nscenes,
+__global__ void __launch_bounds__(kBatchMaxThreads, sizeof(T) == 4 ? 2 : 1) k_batch2d_substeps(unsigned char* ws, PView<T> P, int nscenes,
                                                                         int nsteps) {
   BatchHeader* h = reinterpret_cast<BatchHeader*>(ws);
   __shared__ SceneK<T> s_sc[kMaxScenes];
@@ -329,6 +289,9 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned 
   __shared__ int64_t s_boff[kMaxScenes + 1];
   __shared__ int s_blo0[kMaxScenes], s_blo1[kMaxScenes], s_bw[kMaxScenes];
   __shared__ int s_fail;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  WarpRecs<2, T>& wr = reinterpret_cast<WarpRecs<2, T>*>(smem_raw)[threadIdx.x >> 5];
+  const RunLane<2, T> ln;
   if (nsteps <= 0) return;
   const TableOffsets to = table_offsets(nscenes);
   const SceneK<T>* g_sc = reinterpret_cast<const SceneK<T>*>(ws + to.sk);
@@ -377,7 +340,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned 
       const T e = kp.model == FFMPM_MODEL_SNOW ? ffexp(kp.hardening * (T(1) - P.Jp[p])) : kp.hardening;
       affine_of<2, T>(kp, F, C, kp.mass, kp.mu0 * e, kp.lam0 * e, A2, nullptr);
     }
-    scatter_warp<T>(A, s_noff[si], boxes, si, ok, b, fx, v, A2, kp, lane);
+    scatter_warp<T>(wr, ln, A, s_noff, boxes, si, ok, b, fx, v, A2, kp);
   }
   // (fault injection for tests: CTA 0 never arrives, so the first barrier can only end by running out)
   if ((h->inject & FFMPM_INJECT_BARRIER_ABSENT) && blockIdx.x == 0) return;
@@ -413,15 +376,18 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned 
       const int si = live ? find_scene(s_poff, nscenes, gp) : 0;
       const KParams<T> kp = scene_kparams<T>(s_sc[si]);
       const uint32_t p = (uint32_t)(live ? gp : 0);
-      T xp[2] = {T(0), T(0)}, fx[2] = {T(0), T(0)};
+      T xp[2] = {T(0), T(0)}, fx[2] = {T(0), T(0)}, F[4] = {T(1), T(0), T(0), T(1)}, Jp = T(1);
       int b[2] = {0, 0};
       bool ok = live;
       if (live) {
+        // everything the particle needs from memory in flight together
 #pragma unroll
-        for (int d = 0; d < 2; ++d) {
-          xp[d] = P.x[P.at(p, d, 2)];
-          ok = ok && base_of(xp[d], kp.inv_dx, kp.res, b[d], fx[d]);
-        }
+        for (int d = 0; d < 2; ++d) xp[d] = P.x[P.at(p, d, 2)];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) F[i] = P.F[P.at(p, i, 4)];
+        Jp = P.Jp[p];
+#pragma unroll
+        for (int d = 0; d < 2; ++d) ok = ok && base_of(xp[d], kp.inv_dx, kp.res, b[d], fx[d]);
       }
       T v[2] = {T(0), T(0)}, Cn[4] = {T(0), T(0), T(0), T(0)}, Fn[4] = {T(1), T(0), T(0), T(1)};
       T xn[2] = {T(0), T(0)}, Jpn = T(1);
@@ -461,9 +427,6 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned 
         const T c4 = T(4) * kp.inv_dx;
 #pragma unroll
         for (int i = 0; i < 4; ++i) Cn[i] *= c4;
-        T F[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) F[i] = P.F[P.at(p, i, 4)];
         // F + dt (C F): (I + dt C) F with the increment rounded once against F
         Fn[0] = F[0] + kp.dt * (Cn[0] * F[0] + Cn[1] * F[2]);
         Fn[1] = F[1] + kp.dt * (Cn[0] * F[1] + Cn[1] * F[3]);
@@ -482,22 +445,17 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned 
               Fn[i * 2 + j] = U[i * 2] * s2[0] * V[j * 2] + U[i * 2 + 1] * s2[1] * V[j * 2 + 1];
         }
         const T det = (Fn[0] * Fn[3] - Fn[1] * Fn[2]) + T(1e-10);
-        Jpn = ffclamp(P.Jp[p] * oldJ / det, T(0.6), T(20.0));
+        Jpn = ffclamp(Jp * oldJ / det, T(0.6), T(20.0));
         P.Jp[p] = Jpn;
         xn[0] = xp[0] + kp.dt * v[0];
         xn[1] = xp[1] + kp.dt * v[1];
         if (nonfinite_probe(xn, 2) + nonfinite_probe(Fn, 4) != T(0)) raise_status(&h->status, FFMPM_STATUS_NONFINITE);
 #pragma unroll
-        for (int d = 0; d < 2; ++d) {
-          P.x[P.at(p, d, 2)] = xn[d];
-          P.v[P.at(p, d, 2)] = v[d];
-        }
+        for (int d = 0; d < 2; ++d) P.x[P.at(p, d, 2)] = xn[d];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          P.C[P.at(p, i, 4)] = Cn[i];
-          P.F[P.at(p, i, 4)] = Fn[i];
-        }
+        for (int i = 0; i < 4; ++i) P.F[P.at(p, i, 4)] = Fn[i];
       }
+      bool keep_vc = ok && !next;  // v and C are rebuilt by the next G2P: stored by a particle's last one
       if (next) {  // warp-uniform
         // a particle already outside its grid stays there (G2P left it): its P2G fails as before
         bool ok2 = ok;
@@ -508,12 +466,19 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch2d_substeps(unsigned 
           for (int d = 0; d < 2; ++d) ok2 = ok2 && base_of(xn[d], kp.inv_dx, kp.res, b2[d], fx2[d]);
         }
         if (live && !ok2) raise_status(&h->status, FFMPM_STATUS_OOB);
+        keep_vc = ok && !ok2;
         T A2[4] = {T(0), T(0), T(0), T(0)};
         if (ok2) {
           const T e = kp.model == FFMPM_MODEL_SNOW ? ffexp(kp.hardening * (T(1) - Jpn)) : kp.hardening;
           affine_of<2, T>(kp, Fn, Cn, kp.mass, kp.mu0 * e, kp.lam0 * e, A2, nullptr);
         }
-        scatter_warp<T>(A, s_noff[si], nbox, si, ok2, b2, fx2, v, A2, kp, lane);
+        scatter_warp<T>(wr, ln, A, s_noff, nbox, si, ok2, b2, fx2, v, A2, kp);
+      }
+      if (keep_vc) {
+#pragma unroll
+        for (int d = 0; d < 2; ++d) P.v[P.at(p, d, 2)] = v[d];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) P.C[P.at(p, i, 4)] = Cn[i];
       }
     }
   }
@@ -587,7 +552,13 @@ int ffmpm_batch2d_substeps(int32_t nscenes, int32_t real_bytes, ffmpm_particles*
   const int nt = batch_threads(threads);
   auto launch = [&](auto kern, auto view) -> int {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, 0) != cudaSuccess || per_sm < 1) {
+    const size_t smem = (real_bytes == 4 ? sizeof(WarpRecs<2, float>) : sizeof(WarpRecs<2, double>)) * (nt / 32);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(WarpRecs<2, double>) * (kBatchMaxThreads / 32))) != cudaSuccess) {
+      cudaGetLastError();
+      return FFMPM_ERR_CUDA;
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem) != cudaSuccess || per_sm < 1) {
       cudaGetLastError();
       return FFMPM_ERR_CUDA;
     }
@@ -602,6 +573,7 @@ int ffmpm_batch2d_substeps(int32_t nscenes, int32_t real_bytes, ffmpm_particles*
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

@@ -80,15 +80,29 @@ struct RunLane {
 
 // Sums of the records [l0, l1) of a list grouped by base node (stride kS reals, shared memory) in
 // registers while the base node stays the same, then one vector reduction per node into A.  The
-// bounds may differ from group to group.  A run's momenta are summed relative to its first particle's
-// q / m =: u, sum w (q - m u + a o), and u sum w m is added once at its end: the part that a run has in
-// common so takes no rounding from the run's length.
+// bounds may differ from group to group.  Momenta are summed relative to a velocity u that the list has
+// about in common, sum w (q - m u + a o), and u sum w m is added at the end of a run: the part in common so
+// takes no rounding from the run's length.
 template <int DIM, typename T>
-__device__ __forceinline__ void run_flush(Node4<T>* at, T (&acc)[DIM == 3 ? 3 : 1][4], const T (&u)[DIM], int64_t RR) {
+__device__ __forceinline__ void run_add(Node4<T>* at, const T (&a)[4], const T (&u)[DIM]) {
+  atomic_add4(at, a[0] + u[0] * a[3], a[1] + u[1] * a[3], DIM == 3 ? a[2] + u[DIM - 1] * a[3] : T(0), a[3]);
+}
+template <int DIM, typename T>
+__device__ __forceinline__ void run_flush(Node4<T>* at, const T (&acc)[DIM == 3 ? 3 : 1][4], const T (&u)[DIM],
+                                          int64_t RR) {
 #pragma unroll
-  for (int i = 0; i < (DIM == 3 ? 3 : 1); ++i)
-    atomic_add4(at + i * RR, acc[i][0] + u[0] * acc[i][3], acc[i][1] + u[1] * acc[i][3],
-                DIM == 3 ? acc[i][2] + u[DIM - 1] * acc[i][3] : T(0), acc[i][3]);
+  for (int i = 0; i < (DIM == 3 ? 3 : 1); ++i) run_add<DIM, T>(at + i * RR, acc[i], u);
+}
+
+// q / m of a record, or zero where that is no usable velocity.
+template <int DIM, typename T>
+__device__ __forceinline__ void run_velocity(const T* rec, T (&u)[DIM]) {
+  const T im = rec[0] > T(0) ? ffrcp(rec[0]) : T(0);
+#pragma unroll
+  for (int r = 0; r < DIM; ++r) {
+    const T ur = rec[1 + r] * im;
+    u[r] = ffabs(ur) < T(1e18) ? ur : T(0);
+  }
 }
 
 // A group's sums under way.
@@ -118,8 +132,11 @@ struct RunSums {
   }
 };
 
-// kStages: the list is one of several that a run may go through (put_by between them).
-template <int DIM, typename T, int kS, bool kStages>
+// kStages: the list is one of several that a run may go through (put_by between them), and its records hold
+// q; else they hold q - m u already.  kSlide: keep the sums of shared nodes from cell to cell, which leaves a
+// third of the reductions, so that a node is a sum of fewer parts; it costs 24 shuffles a cell (the
+// resident solver, 16,384 particles: 668 us a call with it, 613 without).
+template <int DIM, typename T, int kS, bool kStages, bool kSlide>
 __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, const int* nodes, int l0, int l1,
                                          const RunLane<DIM, T>& ln, Node4<T>* __restrict__ Al, int64_t RR) {
   constexpr int NX = RunLane<DIM, T>::NX;
@@ -138,24 +155,13 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
     }
     if (nd != rs.cur) {
       if constexpr (kStages) rs.take_up();
-      T u[DIM];
-      const T im = rv[0] > T(0) ? ffrcp(rv[0]) : T(0);
-#pragma unroll
-      for (int r = 0; r < DIM; ++r) {
-        const T ur = rv[1 + r] * im;
-        u[r] = ffabs(ur) < T(1e18) ? ur : T(0);
-      }
-      if (nd == rs.cur + 1 && rs.cur >= 0) {
+      if (kSlide && nd == rs.cur + 1 && rs.cur >= 0) {
         // the next cell along the grid's last axis shares two thirds of the nodes: the sums move one
         // lane down, and only those that no lane holds any more go to the grid
         const unsigned group = 0x1ffu << (9 * ln.grp);
 #pragma unroll
         for (int i = 0; i < NX; ++i) {
-#pragma unroll
-          for (int r = 0; r < DIM; ++r) rs.acc[i][r] += (rs.u[r] - u[r]) * rs.acc[i][3];
-          if (ln.ob == 0)
-            atomic_add4(Al + rs.cur + i * RR, rs.acc[i][0] + u[0] * rs.acc[i][3], rs.acc[i][1] + u[1] * rs.acc[i][3],
-                        DIM == 3 ? rs.acc[i][2] + u[DIM - 1] * rs.acc[i][3] : T(0), rs.acc[i][3]);
+          if (ln.ob == 0) run_add<DIM, T>(Al + rs.cur + i * RR, rs.acc[i], rs.u);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             const T t = __shfl_down_sync(group, rs.acc[i][r], 1);
@@ -167,9 +173,11 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
 #pragma unroll
         for (int i = 0; i < NX; ++i) rs.acc[i][0] = rs.acc[i][1] = rs.acc[i][2] = rs.acc[i][3] = T(0);
       }
-#pragma unroll
-      for (int r = 0; r < DIM; ++r) rs.u[r] = u[r];
       rs.cur = nd;
+    }
+    if constexpr (kStages) {
+#pragma unroll
+      for (int r = 0; r < DIM; ++r) rv[1 + r] -= rv[0] * rs.u[r];
     }
     if constexpr (DIM == 3) {
       const T da = rv[f0 + 1] - ln.ra, db = rv[f0 + 2] - ln.rb;
@@ -179,7 +187,7 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
       T b[3];
 #pragma unroll
       for (int r = 0; r < 3; ++r)
-        b[r] = (rv[1 + r] - rv[0] * rs.u[r]) + rv[a0 + 3 * r + 1] * T(ln.oa) + rv[a0 + 3 * r + 2] * T(ln.ob);
+        b[r] = rv[1 + r] + rv[a0 + 3 * r + 1] * T(ln.oa) + rv[a0 + 3 * r + 2] * T(ln.ob);
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         const T wt = wx[i] * wjk;
@@ -192,7 +200,7 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
       const T wt = (ln.ka * da * da + ln.ea) * (ln.kb * db * db + ln.eb);
 #pragma unroll
       for (int r = 0; r < 2; ++r)
-        rs.acc[0][r] += wt * ((rv[1 + r] - rv[0] * rs.u[r]) + rv[a0 + 2 * r] * T(ln.oa) + rv[a0 + 2 * r + 1] * T(ln.ob));
+        rs.acc[0][r] += wt * (rv[1 + r] + rv[a0 + 2 * r] * T(ln.oa) + rv[a0 + 2 * r + 1] * T(ln.ob));
       rs.acc[0][3] += wt * rv[0];
     }
   }
@@ -242,13 +250,23 @@ struct alignas(16) WarpRecs {
 };
 
 template <int DIM, typename T>
-__device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec)[RunRec<DIM>::kPacked], int node,
+__device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec_in)[RunRec<DIM>::kPacked], int node,
                                              const RunLane<DIM, T>& ln, Node4<T>* __restrict__ A, int R) {
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const bool valid = node >= 0;
   const unsigned vmask = __ballot_sync(kFull, valid);
   if (vmask == 0u) return;
+  RunSums<DIM, T> rs;
+  run_velocity<DIM, T>(rec_in, rs.u);
+  T rec[RunRec<DIM>::kPacked];
+#pragma unroll
+  for (int i = 0; i < RunRec<DIM>::kPacked; ++i) rec[i] = rec_in[i];
+#pragma unroll
+  for (int r = 0; r < DIM; ++r) {
+    rs.u[r] = __shfl_sync(kFull, rs.u[r], __ffs(vmask) - 1);
+    rec[1 + r] -= rec[0] * rs.u[r];
+  }
   // slot of the lane's record: the lanes of one base node together, groups in order of first lane
   const unsigned peers = __match_any_sync(kFull, node);
   const unsigned before = peers & lanemask_lt();
@@ -274,8 +292,7 @@ __device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec
   const int l0 = ln.grp * per;
   const int64_t RR = DIM == 3 ? (int64_t)R * R : 0;
   Node4<T>* const Al = A + (ln.oa * R + ln.ob);
-  RunSums<DIM, T> rs;
-  run_sums<DIM, T, RunRec<DIM>::kSmem, false>(rs, &wr.rec[0][0], wr.node, l0, ln.grp < 3 ? min(nv, l0 + per) : 0, ln, Al, RR);
+  run_sums<DIM, T, RunRec<DIM>::kSmem, false, false>(rs, &wr.rec[0][0], wr.node, l0, ln.grp < 3 ? min(nv, l0 + per) : 0, ln, Al, RR);
   run_end<DIM, T>(rs, ln, Al, RR);
   __syncwarp();  // the records are rewritten by the warp's next particles
 }
@@ -500,7 +517,8 @@ __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ r
     fetch(k);
     __syncwarp();
     const int l0 = kPitch * min(ln.grp, 2);
-    run_sums<DIM, T, kS, true>(rs, &ws.rec[0][0], ws.node, l0, l0 + max(0, min(32, my_len - 32 * k)), ln, Al, RR);
+    if (k == 0 && my_len > 0) run_velocity<DIM, T>(ws.rec[l0], rs.u);
+    run_sums<DIM, T, kS, true, true>(rs, &ws.rec[0][0], ws.node, l0, l0 + max(0, min(32, my_len - 32 * k)), ln, Al, RR);
     rs.put_by();
     __syncwarp();
   }
@@ -581,9 +599,9 @@ __global__ void __launch_bounds__(kWarpCta<T>) k_g2p_range(KParams<T> kp, Geom<D
 // cells, its scatter is warp_scatter's (the particles that crossed a cell boundary since the last re-sort
 // join the run of their new cell there).  The grid update visits the blocks the plan touches: a
 // particle whose new stencil may leave them adds the blocks it covers to the list itself.
-// Two cubes of 1,048,576 particles on 128^3 (GB300): 122 us a launch; chunks of 512 particles with a
+// Two cubes of 1,048,576 particles on 128^3 (GB300): 115 us a launch; chunks of 512 particles with a
 // shared-memory tile for each side, an in-chunk counting sort and CTA barriers between the phases took
-// 156.  16,384 particles on 64^3: 13 us a substep against 38 (512 one-warp batches instead of 32 chunks).
+// 156.  16,384 particles on 64^3: 13 us a substep against 40 (512 one-warp batches instead of 32 chunks).
 // Bound by instruction issue and the latency of the gathers.
 
 // Add the blocks covered by the stencil at `base` to the touched list (each block once: `tmark` is
