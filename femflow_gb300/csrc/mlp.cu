@@ -1,5 +1,5 @@
 // BF16 tensor-core kernels of the learned corrector (tcgen05 MMA, FP32 accumulation in tensor
-// memory).  This file holds the general GEMM used by training; the fused per-particle inference
+// memory).  This file holds a general GEMM and the training kernels; the fused per-particle inference
 // kernel lives in corrector.cu.
 //
 // k_tc_gemm: D[M][N] = A[M][K] . B[N][K]^T, bf16 operands row-major in global memory, float32 D.
@@ -145,85 +145,372 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.3989422804014327f * expf(-0.5f * z * z);
 }
 
-// Z (float [B][N]) += bias, kept for the backward pass; H = act(Z) as bf16 [B][N] and, when Ht is
-// given, its transpose [N][B].
-__global__ void __launch_bounds__(kEw) k_bias_act(float* __restrict__ Z, const float* __restrict__ bias, int B, int N,
-                                                  int act, uint16_t* __restrict__ H, uint16_t* __restrict__ Ht) {
-  const int64_t i = (int64_t)blockIdx.x * kEw + threadIdx.x;
-  if (i >= (int64_t)B * N) return;
-  const int row = (int)(i / N), col = (int)(i % N);
-  const float z = Z[i] + bias[col];
-  Z[i] = z;
-  const uint16_t h = tc::bf16_bits(act ? gelu_f(z) : z);
-  H[i] = h;
-  if (Ht) Ht[(size_t)col * B + row] = h;
+// ---------------------------------------------------------------------------------------------
+// Forward and backward of the whole network, a tile of 128 rows at a time.  A CTA has 256 threads:
+// thread t works on row t & 127 (its TMEM lane) and on one half of a layer's 64 columns (t >> 7).
+// 32,768 rows (GB300): 45 + 64 us, and 117 us for a whole training step; a launch for each GEMM and each
+// elementwise part, with transposes written a 16-bit word at a time, took 777.  Bound by the chain of a
+// tile's layers (an MMA, its commit, the activation), two CTAs (forward) or one (backward) per SM.
+constexpr int kTrain = 256;
+constexpr uint32_t kSbo64 = (64 / 8) * 128, kSbo128 = (128 / 8) * 128;
+
+// Copy a bf16 row-major [rows][k] matrix (row stride k) into the K-major core-matrix layout.
+__device__ __forceinline__ void stage_kmajor(unsigned char* dst, const uint16_t* src, int rows, int k, uint32_t sbo) {
+  const int vecs = k / 8;
+  for (int v = threadIdx.x; v < rows * vecs; v += blockDim.x) {
+    const int r = v / vecs, c = v - r * vecs;
+    *reinterpret_cast<uint4*>(dst + tc::kmajor_offset(r, 8 * c, sbo)) =
+        *reinterpret_cast<const uint4*>(src + (size_t)r * k + 8 * c);
+  }
 }
 
-// X [B][K] -> Xt [K][B] (bf16); rows k >= kmax of Xt are zeroed (the buffer is strided by B).
-__global__ void __launch_bounds__(kEw) k_transpose_bf16(const uint16_t* __restrict__ X, int B, int K, int kmax,
-                                                        uint16_t* __restrict__ Xt) {
-  const int64_t i = (int64_t)blockIdx.x * kEw + threadIdx.x;
-  if (i >= (int64_t)B * K) return;
-  const int row = (int)(i / K), col = (int)(i % K);
-  Xt[(size_t)col * B + row] = col < kmax ? X[(size_t)row * K + col] : uint16_t(0);
+// The transpose of a K-major tile [128 rows][cols] as rows of a bf16 matrix [cols][B]: out[c][r0 + r], two
+// rows per 32-bit store, columns from `valid` on as zeros.
+__device__ __forceinline__ void store_transposed(const unsigned char* tile, uint32_t sbo, int cols, int valid,
+                                                 uint16_t* __restrict__ out, int B, int r0) {
+  for (int i = threadIdx.x; i < cols * 64; i += blockDim.x) {
+    const int c = i >> 6, r = 2 * (i & 63);
+    uint32_t w = 0u;
+    if (c < valid)
+      w = uint32_t(*reinterpret_cast<const uint16_t*>(tile + tc::kmajor_offset(r, c, sbo))) |
+          (uint32_t(*reinterpret_cast<const uint16_t*>(tile + tc::kmajor_offset(r + 1, c, sbo))) << 16);
+    *reinterpret_cast<uint32_t*>(out + (size_t)c * B + r0 + r) = w;
+  }
 }
 
-// Weighted squared error of Y (+ b4) against T; dY = 2 w (pred - T) / B as bf16 [B][64] (zero beyond
-// 12) and its transpose [12..][B]; db4 += column sums; *loss += the loss.
-__global__ void __launch_bounds__(kEw) k_loss_grad(const float* __restrict__ Y, const float* __restrict__ b4,
-                                                   const float* __restrict__ T, const float* __restrict__ w, int B,
-                                                   uint16_t* __restrict__ dY, uint16_t* __restrict__ dYt,
-                                                   float* __restrict__ db4, double* __restrict__ loss) {
-  __shared__ float s_db[FFMPM_MLP_OUT];
-  __shared__ double s_loss;
-  if (threadIdx.x < FFMPM_MLP_OUT) s_db[threadIdx.x] = 0.f;
-  if (threadIdx.x == 0) s_loss = 0.0;
+// D (+)= A . B^T over K = 16 ksteps, both operands K-major tiles.
+__device__ __forceinline__ void mma_tile(uint32_t d, const unsigned char* A, uint32_t sboA, const unsigned char* B,
+                                         uint32_t sboB, uint32_t idesc, int ksteps, bool accumulate) {
+  const uint32_t a0 = tc::smem_addr(A), b0 = tc::smem_addr(B);
+  for (int s = 0; s < ksteps; ++s)
+    tc::mma_bf16(d, tc::make_desc(a0 + 256u * s, tc::kLBO, sboA), tc::make_desc(b0 + 256u * s, tc::kLBO, sboB), idesc,
+                 accumulate || s > 0);
+}
+
+// Four floats at p, whole where the caller's arrays are 16-byte aligned (`vec`), else one by one.
+__device__ __forceinline__ float4 load4(const float* p, bool vec) {
+  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ void store4(float* p, float4 v, bool vec) {
+  if (vec) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    p[0] = v.x;
+    p[1] = v.y;
+    p[2] = v.z;
+    p[3] = v.w;
+  }
+}
+__device__ __forceinline__ void add4(float* p, float4 v, bool vec) {
+  if (vec) {
+    atomicAdd(reinterpret_cast<float4*>(p), v);
+  } else {
+    atomicAdd(p, v.x);
+    atomicAdd(p + 1, v.y);
+    atomicAdd(p + 2, v.z);
+    atomicAdd(p + 3, v.w);
+  }
+}
+
+struct FwdSmem {
+  static constexpr size_t w1 = 0, w2 = w1 + 64 * 128 * 2, w3 = w2 + 64 * 64 * 2, w4 = w3 + 64 * 64 * 2,
+                          x = w4 + 16 * 64 * 2, h = x + 128 * 128 * 2, bias = h + 128 * 64 * 2,
+                          total = bias + 3 * 64 * 4;
+};
+
+// Y = network(X) (before out_scale, without b4).  Keeps Z1..Z3 (with the biases), H1..H3 = gelu(Z) and the
+// transposes Ht and Xt, as the ABI documents; the backward pass reads X, Z and H.  One CTA per 128 rows:
+// the layers follow one another in shared and tensor memory (an MMA a layer), so that X is read once and
+// everything is written once.
+__global__ void __launch_bounds__(kTrain) k_mlp_forward(ffmpm_mlp_trainer t, const uint16_t* __restrict__ X, int B,
+                                                        bool vec) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char *sX = smem + FwdSmem::x, *sH = smem + FwdSmem::h;
+  float* sbias = reinterpret_cast<float*>(smem + FwdSmem::bias);
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_base;
+  __shared__ int s_fail;
+  const int tid = threadIdx.x, warp = tid >> 5, row = tid & 127, c0 = 32 * (tid >> 7);
+  const uint32_t lanes = 32u * (warp & 3);
+  const int r0 = blockIdx.x * 128;
+  stage_kmajor(sX, X + (size_t)r0 * FFMPM_MLP_IN, 128, FFMPM_MLP_IN, kSbo128);
+  stage_kmajor(smem + FwdSmem::w1, t.W1, 64, 128, kSbo128);
+  stage_kmajor(smem + FwdSmem::w2, t.W2, 64, 64, kSbo64);
+  stage_kmajor(smem + FwdSmem::w3, t.W3, 64, 64, kSbo64);
+  stage_kmajor(smem + FwdSmem::w4, t.W4, 16, 64, kSbo64);
+  if (tid < 192) sbias[tid] = t.params[FFMPM_MLP_OFF_B1 + tid];  // b1, b2, b3 lie one after another
+  if (warp == 0) tc::tmem_alloc(&tmem_base, 128);
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+    s_fail = 0;
+  }
+  fence_proxy_async_shared();
+  tc::fence_before_sync();
   __syncthreads();
-  const int row = blockIdx.x * kEw + threadIdx.x;
-  double l = 0.0;
-  if (row < B) {
-    const float invB = 1.f / float(B);
-#pragma unroll
-    for (int j = 0; j < FFMPM_MLP_OUT; ++j) {
-      const float e = Y[(size_t)row * 16 + j] + b4[j] - T[(size_t)row * FFMPM_MLP_OUT + j];
-      l += double(w[j]) * double(e) * double(e);
-      const float g = 2.f * w[j] * e * invB;
-      const uint16_t gb = tc::bf16_bits(g);
-      dY[(size_t)row * 64 + j] = gb;
-      dYt[(size_t)j * B + row] = gb;
-      atomicAdd(&s_db[j], g);
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_base;
+  uint32_t phase = 0;
+  float* const Zs[3] = {t.Z1, t.Z2, t.Z3};
+  uint16_t* const Hs[3] = {t.H1, t.H2, t.H3};
+  uint16_t* const Hts[3] = {t.H1t, t.H2t, t.H3t};
+#pragma unroll 1
+  for (int layer = 0; layer < 4; ++layer) {
+    if (tid == 0) {
+      const size_t wo = layer == 0 ? FwdSmem::w1 : layer == 1 ? FwdSmem::w2 : layer == 2 ? FwdSmem::w3 : FwdSmem::w4;
+      if (layer == 0)
+        mma_tile(tmem, sX, kSbo128, smem + wo, kSbo128, tc::idesc_bf16_f32(128, 64), 8, false);
+      else
+        mma_tile(tmem + (layer == 3 ? 64u : 0u), sH, kSbo64, smem + wo, kSbo64,
+                 layer == 3 ? tc::idesc_bf16_f32(128, 16) : tc::idesc_bf16_f32(128, 64), 4, false);
+      tc::commit(&bar);
     }
+    // while the tensor core works: the transpose of the layer's input
+    if (layer == 0)
+      store_transposed(sX, kSbo128, 128, FFMPM_MLP_FEATURES, t.Xt, B, r0);
+    else
+      store_transposed(sH, kSbo64, 64, 64, Hts[layer - 1], B, r0);
+    if (!mbar_wait(&bar, phase)) s_fail = 1;
+    phase ^= 1u;
+    tc::fence_after_sync();
+    __syncthreads();  // also: every thread has read sH
+    if (s_fail) break;
+    if (layer < 3) {
+#pragma unroll 1
+      for (int c = c0; c < c0 + 32; c += 16) {
+        float a[16];
+        tc::tmem_ld16(tc::taddr_of(tmem, lanes, c), a);
+        uint32_t hw[8];
 #pragma unroll
-    for (int j = FFMPM_MLP_OUT; j < 64; ++j) dY[(size_t)row * 64 + j] = 0;
-    for (int j = FFMPM_MLP_OUT; j < 128; ++j) dYt[(size_t)j * B + row] = 0;  // padding rows of the transpose
+        for (int j = 0; j < 16; ++j) a[j] += sbias[64 * layer + c + j];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          hw[j] = uint32_t(tc::bf16_bits(gelu_f(a[2 * j]))) | (uint32_t(tc::bf16_bits(gelu_f(a[2 * j + 1]))) << 16);
+        const size_t at = (size_t)(r0 + row) * 64 + c;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          store4(Zs[layer] + at + 4 * j, make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]), vec);
+        uint4* h = reinterpret_cast<uint4*>(Hs[layer] + at);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint4 v = make_uint4(hw[4 * j], hw[4 * j + 1], hw[4 * j + 2], hw[4 * j + 3]);
+          h[j] = v;
+          *reinterpret_cast<uint4*>(sH + tc::kmajor_offset(row, c + 8 * j, kSbo64)) = v;
+        }
+      }
+      fence_proxy_async_shared();
+      tc::fence_before_sync();
+      __syncthreads();
+      tc::fence_after_sync();
+    } else if (c0 == 0) {
+      float y[16];
+      tc::tmem_ld16(tc::taddr_of(tmem, lanes, 64), y);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        store4(t.Y + (size_t)(r0 + row) * 16 + 4 * j, make_float4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]),
+               vec);
+    }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(&s_loss, l);
+  if (s_fail && tid == 0) {
+    if (t.status) raise_status(t.status, FFMPM_STATUS_TIMEOUT);
+    // the MMAs of the last commit may still be running: wait for them once more (bounded) before
+    // their tensor memory is freed
+    mbar_wait(&bar, phase ^ 1u);
+  }
+  tc::fence_before_sync();
   __syncthreads();
-  if (threadIdx.x < FFMPM_MLP_OUT) atomicAdd(&db4[threadIdx.x], s_db[threadIdx.x]);
-  if (threadIdx.x == 0) atomicAdd(loss, s_loss / double(B));
+  if (warp == 0) tc::tmem_free(tmem, 128);
 }
 
-// dZ = dH * GELU'(Z) as bf16 [B][64] and transpose [64..][B]; db += column sums.
-__global__ void __launch_bounds__(kEw) k_act_back(const float* __restrict__ dH, const float* __restrict__ Z, int B,
-                                                  uint16_t* __restrict__ dZ, uint16_t* __restrict__ dZt,
-                                                  float* __restrict__ db) {
-  __shared__ float s_db[64];
-  if (threadIdx.x < 64) s_db[threadIdx.x] = 0.f;
-  __syncthreads();
-  const int64_t i = (int64_t)blockIdx.x * kEw + threadIdx.x;
-  if (i < (int64_t)B * 64) {
-    const int row = (int)(i >> 6), col = (int)(i & 63);
-    const float g = dH[i] * gelu_grad(Z[i]);
-    const uint16_t gb = tc::bf16_bits(g);
-    dZ[i] = gb;
-    dZt[(size_t)col * B + row] = gb;
-    dZt[(size_t)(col + 64) * B + row] = 0;  // padding rows 64..127 of the transpose
-    atomicAdd(&s_db[col], g);
+// Tensor-memory columns of the backward pass: the gradients of the four weight matrices (row = output
+// unit) and the adjoint of a layer's input.
+constexpr uint32_t kColW1 = 0, kColW2 = 128, kColW3 = 192, kColW4 = 256, kColDH = 320;
+struct BwdSmem {
+  static constexpr size_t w4t = 0, w3t = w4t + 64 * 64 * 2, w2t = w3t + 64 * 64 * 2,
+                          g = w2t + 64 * 64 * 2,     // dY / dZ [128 rows][64]
+                          gt = g + 128 * 64 * 2,     // its transpose [128: 64 used][128 rows]
+                          it = gt + 128 * 128 * 2,   // transpose of the layer's input [up to 128][128 rows]
+                          used = it + 128 * 128 * 2;
+  // one CTA per SM: each holds all 512 tensor-memory columns
+  static constexpr size_t total = used > 120 * 1024 ? used : 120 * 1024;
+};
+
+// Two neighbouring columns c (even), c + 1 of the thread's row into the transposed tile [c][row]: the lanes
+// of two neighbouring rows swap a value, so that each stores one 32-bit word.
+__device__ __forceinline__ void put_transposed2(unsigned char* tile, int c, int row, uint32_t lo, uint32_t hi) {
+  const bool odd = row & 1;
+  const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+  const uint32_t w = odd ? (got | (hi << 16)) : (lo | (got << 16));
+  *reinterpret_cast<uint32_t*>(tile + tc::kmajor_offset(c + (odd ? 1 : 0), row & ~1, kSbo128)) = w;
+}
+
+// Sum over the warp's 32 rows of 32 columns: lane l returns the sum of column l.
+__device__ __forceinline__ float column_sum(float (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const bool up = lane & o;
+      const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  return v[0];
+}
+
+// Loss and the gradient of every parameter (added to zeroed grads).  Per tile of 128 rows and layer, from
+// the last to the first: g = dL/d(layer's output) in bf16, then on the tensor cores the adjoint of the
+// layer's input, g . W, and the layer's weight gradient, g^T . input, whose accumulator stays in tensor
+// memory over all the tiles of the CTA.
+__global__ void __launch_bounds__(kTrain) k_mlp_backward(ffmpm_mlp_trainer t, const float* __restrict__ T,
+                                                         const float* __restrict__ w, int B,
+                                                         double* __restrict__ loss, bool vec) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char *sG = smem + BwdSmem::g, *sGt = smem + BwdSmem::gt, *sIt = smem + BwdSmem::it;
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_base;
+  __shared__ int s_fail;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = tid & 127, c0 = 32 * (tid >> 7);
+  const uint32_t lanes = 32u * (warp & 3);
+  stage_kmajor(smem + BwdSmem::w4t, t.W4t, 64, 64, kSbo64);
+  stage_kmajor(smem + BwdSmem::w3t, t.W3t, 64, 64, kSbo64);
+  stage_kmajor(smem + BwdSmem::w2t, t.W2t, 64, 64, kSbo64);
+  for (int i = tid; i < 128 * 128 * 2 / 16; i += kTrain) reinterpret_cast<uint4*>(sGt)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+    s_fail = 0;
   }
+  tc::fence_before_sync();
   __syncthreads();
-  if (threadIdx.x < 64) atomicAdd(&db[threadIdx.x], s_db[threadIdx.x]);
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_base;
+  uint32_t phase = 0;
+  bool first = true;
+  double l = 0.0;
+  float db[4] = {0.f, 0.f, 0.f, 0.f};  // column c0 + lane of b1..b4, over the warp's rows
+  const float* const Zs[3] = {t.Z1, t.Z2, t.Z3};
+  const uint16_t* const ins[4] = {t.Xt, t.H1t, t.H2t, t.H3t};  // the layers' inputs, transposed [width][B]
+  const float* const b4 = t.params + FFMPM_MLP_OFF_B4;
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile * 128 < B; tile += gridDim.x) {
+    const size_t r = (size_t)tile * 128 + row;
+#pragma unroll 1
+    for (int layer = 3; layer >= 0; --layer) {
+      float g[32];  // dL/d(output of the layer before its activation), the thread's columns
+      if (layer == 3) {
+        const float invB = 1.f / float(B);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) g[j] = 0.f;
+        if (c0 == 0) {
+#pragma unroll
+          for (int j = 0; j < FFMPM_MLP_OUT; ++j) {
+            const float e = t.Y[r * 16 + j] + b4[j] - T[r * FFMPM_MLP_OUT + j];
+            l += double(w[j]) * double(e) * double(e);
+            g[j] = 2.f * w[j] * e * invB;
+          }
+        }
+      } else {
+        const float* z = Zs[layer] + r * 64 + c0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float a[16];
+          tc::tmem_ld16(tc::taddr_of(tmem, lanes, kColDH + c0 + 16 * h), a);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 zz = load4(z + 16 * h + 4 * j, vec);
+            g[16 * h + 4 * j] = a[4 * j] * gelu_grad(zz.x);
+            g[16 * h + 4 * j + 1] = a[4 * j + 1] * gelu_grad(zz.y);
+            g[16 * h + 4 * j + 2] = a[4 * j + 2] * gelu_grad(zz.z);
+            g[16 * h + 4 * j + 3] = a[4 * j + 3] * gelu_grad(zz.w);
+          }
+        }
+      }
+      // g as the operand of g . W (layer > 0) and, transposed, of g^T . input
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+        uint32_t q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t lo = tc::bf16_bits(g[j + 2 * k]), hi = tc::bf16_bits(g[j + 2 * k + 1]);
+          q[k] = lo | (hi << 16);
+          put_transposed2(sGt, c0 + j + 2 * k, row, lo, hi);
+        }
+        if (layer > 0)
+          *reinterpret_cast<uint4*>(sG + tc::kmajor_offset(row, c0 + j, kSbo64)) = make_uint4(q[0], q[1], q[2], q[3]);
+      }
+      // the layer's input: 128 columns of its transpose (rows 113.. of Xt are zero: those features take no
+      // gradient)
+      {
+        const uint16_t* in = ins[layer] + (size_t)tile * 128;
+        const int width = layer > 0 ? 64 : 128;
+        for (int v = tid; v < width * 16; v += kTrain) {
+          const int c = v >> 4, q = 8 * (v & 15);
+          *reinterpret_cast<uint4*>(sIt + tc::kmajor_offset(c, q, kSbo128)) =
+              *reinterpret_cast<const uint4*>(in + (size_t)c * B + q);
+        }
+      }
+      db[layer] += column_sum(g);
+      fence_proxy_async_shared();
+      tc::fence_before_sync();
+      __syncthreads();
+      tc::fence_after_sync();
+      if (tid == 0) {
+        if (layer > 0) {
+          const size_t wt = layer == 3 ? BwdSmem::w4t : layer == 2 ? BwdSmem::w3t : BwdSmem::w2t;
+          mma_tile(tmem + kColDH, sG, kSbo64, smem + wt, kSbo64, tc::idesc_bf16_f32(128, 64), 4, false);
+        }
+        const uint32_t col = layer == 3 ? kColW4 : layer == 2 ? kColW3 : layer == 1 ? kColW2 : kColW1;
+        mma_tile(tmem + col, sGt, kSbo128, sIt, kSbo128, tc::idesc_bf16_f32(128, layer > 0 ? 64 : 128), 8, !first);
+        tc::commit(&bar);
+      }
+      if (!mbar_wait(&bar, phase)) s_fail = 1;
+      phase ^= 1u;
+      tc::fence_after_sync();
+      __syncthreads();
+      if (s_fail) break;
+    }
+    if (s_fail) break;
+    first = false;
+  }
+  if (s_fail) {
+    if (tid == 0) {
+      if (t.status) raise_status(t.status, FFMPM_STATUS_TIMEOUT);
+      mbar_wait(&bar, phase ^ 1u);
+    }
+  } else if (!first) {
+    float* G = t.grads;
+    // the weight gradients: row = lane of tensor memory (64 used, 12 for W4), the columns split over the halves
+    const int out = row;
+    const auto add = [&](uint32_t col, int cols, int off, int ld, int rows) {
+#pragma unroll 1
+      for (int c = (tid >> 7) * (cols / 2); c < ((tid >> 7) + 1) * (cols / 2); c += 16) {
+        float a[16];
+        tc::tmem_ld16(tc::taddr_of(tmem, lanes, col + c), a);
+        if (out < rows) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            add4(G + off + (size_t)out * ld + c + 4 * j,
+                 make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]), vec);
+        }
+      }
+    };
+    add(kColW1, 128, FFMPM_MLP_OFF_W1, 128, 64);
+    add(kColW2, 64, FFMPM_MLP_OFF_W2, 64, 64);
+    add(kColW3, 64, FFMPM_MLP_OFF_W3, 64, 64);
+    add(kColW4, 64, FFMPM_MLP_OFF_W4, 64, FFMPM_MLP_OUT);
+    atomicAdd(&G[FFMPM_MLP_OFF_B1 + c0 + lane], db[0]);
+    atomicAdd(&G[FFMPM_MLP_OFF_B2 + c0 + lane], db[1]);
+    atomicAdd(&G[FFMPM_MLP_OFF_B3 + c0 + lane], db[2]);
+    if (c0 == 0 && lane < FFMPM_MLP_OUT) atomicAdd(&G[FFMPM_MLP_OFF_B4 + lane], db[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0 && c0 == 0) atomicAdd(loss, l / double(B));
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
 __global__ void __launch_bounds__(kEw) k_adam(float* __restrict__ p, const float* __restrict__ g,
@@ -259,10 +546,19 @@ __global__ void __launch_bounds__(kEw) k_pack(const float* __restrict__ P, uint1
 
 int ew_grid(int64_t n) { return (int)((n + kEw - 1) / kEw); }
 
-int gemm(const uint16_t* A, const uint16_t* B, float* D, int M, int N, int K, int split, int32_t* st, cudaStream_t s) {
-  if (N <= 16) return launch_gemm<16>(A, B, D, M, N, K, split, st, s);
-  if (N <= 64) return launch_gemm<64>(A, B, D, M, N, K, split, st, s);
-  return launch_gemm<128>(A, B, D, M, N, K, split, st, s);
+// Whether the float buffers that the training kernels access four floats at a time are 16-byte aligned (the
+// bf16 ones have to be).
+bool aligned16(const ffmpm_mlp_trainer& t) {
+  return ((reinterpret_cast<uintptr_t>(t.Z1) | reinterpret_cast<uintptr_t>(t.Z2) | reinterpret_cast<uintptr_t>(t.Z3) |
+           reinterpret_cast<uintptr_t>(t.Y) | reinterpret_cast<uintptr_t>(t.grads)) & 15) == 0;
+}
+
+// Raise a kernel's dynamic shared-memory limit (once: `done`).
+template <typename F>
+void allow_smem(F* kern, size_t bytes, bool* done) {
+  if (*done) return;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  *done = true;
 }
 
 }  // namespace
@@ -288,18 +584,9 @@ int ffmpm_tc_gemm_bf16(const uint16_t* A, const uint16_t* B, float* D, int32_t M
 
 int ffmpm_mlp_train_forward(const ffmpm_mlp_trainer* t, const uint16_t* X, int32_t B, void* stream) {
   if (!t || !X || B <= 0 || B % 128 || B > t->max_batch || (reinterpret_cast<uintptr_t>(X) & 15)) return FFMPM_ERR_BADARG;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const float* P = t->params;
-  int rc = FFMPM_OK;
-  k_transpose_bf16<<<ew_grid((int64_t)B * FFMPM_MLP_IN), kEw, 0, s>>>(X, B, FFMPM_MLP_IN, FFMPM_MLP_FEATURES, t->Xt);
-  rc |= gemm(X, t->W1, t->Z1, B, 64, FFMPM_MLP_IN, 1, t->status, s);
-  k_bias_act<<<ew_grid((int64_t)B * 64), kEw, 0, s>>>(t->Z1, P + FFMPM_MLP_OFF_B1, B, 64, 1, t->H1, t->H1t);
-  rc |= gemm(t->H1, t->W2, t->Z2, B, 64, 64, 1, t->status, s);
-  k_bias_act<<<ew_grid((int64_t)B * 64), kEw, 0, s>>>(t->Z2, P + FFMPM_MLP_OFF_B2, B, 64, 1, t->H2, t->H2t);
-  rc |= gemm(t->H2, t->W3, t->Z3, B, 64, 64, 1, t->status, s);
-  k_bias_act<<<ew_grid((int64_t)B * 64), kEw, 0, s>>>(t->Z3, P + FFMPM_MLP_OFF_B3, B, 64, 1, t->H3, t->H3t);
-  rc |= gemm(t->H3, t->W4, t->Y, B, 16, 64, 1, t->status, s);
-  if (rc != FFMPM_OK) return FFMPM_ERR_CUDA;
+  static bool allowed = false;
+  allow_smem(k_mlp_forward, FwdSmem::total, &allowed);
+  k_mlp_forward<<<B / 128, kTrain, FwdSmem::total, static_cast<cudaStream_t>(stream)>>>(*t, X, B, aligned16(*t));
   return cudaGetLastError() == cudaSuccess ? FFMPM_OK : FFMPM_ERR_CUDA;
 }
 
@@ -307,27 +594,10 @@ int ffmpm_mlp_train_backward(const ffmpm_mlp_trainer* t, const float* T, const f
                              void* stream) {
   if (!t || !T || !w || !loss || B <= 0 || B % 128 || B > t->max_batch) return FFMPM_ERR_BADARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  float* G = t->grads;
-  const float* P = t->params;
-  const int split = std::max(1, std::min(2 * sm_count(), B / 1024));
-  int rc = FFMPM_OK;
-  cudaMemsetAsync(G, 0, sizeof(float) * FFMPM_MLP_PARAMS, s);
-  k_loss_grad<<<ew_grid(B), kEw, 0, s>>>(t->Y, P + FFMPM_MLP_OFF_B4, T, w, B, t->dY, t->dYt, G + FFMPM_MLP_OFF_B4, loss);
-  // layer 4: dW4 = dY^T H3, dH3 = dY W4
-  rc |= gemm(t->dYt, t->H3t, G + FFMPM_MLP_OFF_W4, 128, 64, B, split, t->status, s);
-  rc |= gemm(t->dY, t->W4t, t->dH, B, 64, 64, 1, t->status, s);
-  k_act_back<<<ew_grid((int64_t)B * 64), kEw, 0, s>>>(t->dH, t->Z3, B, t->dZ, t->dZt, G + FFMPM_MLP_OFF_B3);
-  // layer 3
-  rc |= gemm(t->dZt, t->H2t, G + FFMPM_MLP_OFF_W3, 128, 64, B, split, t->status, s);
-  rc |= gemm(t->dZ, t->W3t, t->dH, B, 64, 64, 1, t->status, s);
-  k_act_back<<<ew_grid((int64_t)B * 64), kEw, 0, s>>>(t->dH, t->Z2, B, t->dZ, t->dZt, G + FFMPM_MLP_OFF_B2);
-  // layer 2
-  rc |= gemm(t->dZt, t->H1t, G + FFMPM_MLP_OFF_W2, 128, 64, B, split, t->status, s);
-  rc |= gemm(t->dZ, t->W2t, t->dH, B, 64, 64, 1, t->status, s);
-  k_act_back<<<ew_grid((int64_t)B * 64), kEw, 0, s>>>(t->dH, t->Z1, B, t->dZ, t->dZt, G + FFMPM_MLP_OFF_B1);
-  // layer 1: dW1 = dZ1^T X
-  rc |= gemm(t->dZt, t->Xt, G + FFMPM_MLP_OFF_W1, 128, 128, B, split, t->status, s);
-  if (rc != FFMPM_OK) return FFMPM_ERR_CUDA;
+  static bool allowed = false;
+  allow_smem(k_mlp_backward, BwdSmem::total, &allowed);
+  cudaMemsetAsync(t->grads, 0, sizeof(float) * FFMPM_MLP_PARAMS, s);
+  k_mlp_backward<<<std::min(B / 128, sm_count()), kTrain, BwdSmem::total, s>>>(*t, T, w, B, loss, aligned16(*t));
   return cudaGetLastError() == cudaSuccess ? FFMPM_OK : FFMPM_ERR_CUDA;
 }
 
