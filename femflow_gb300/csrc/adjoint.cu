@@ -34,6 +34,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "mpm_kernels.cuh"
+#include "warp_kernels.cuh"
 
 namespace ffmpm {
 namespace {
@@ -109,6 +110,12 @@ __device__ __forceinline__ void store_node(Node4<double>* g, int64_t i, double x
   g[i] = Node4<double>{x, y, z, w};
 }
 
+template <typename G>
+__device__ __forceinline__ void store_zero(G* g, int64_t i) {
+  uint4* p = reinterpret_cast<uint4*>(g + i);  // 32 bytes in either format
+  p[0] = p[1] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Node value minus the reference node value c, per component.
 __device__ __forceinline__ void node_dev(const HiLo4& a, const HiLo4& c, float o[4]) {
   o[0] = (a.hi.x - c.hi.x) + (a.lo.x - c.lo.x);
@@ -132,6 +139,165 @@ __device__ __forceinline__ void red_add3(Node4<double>* p, double a, double b, d
   atomicAdd(&p->x, a);
   atomicAdd(&p->y, b);
   atomicAdd(&p->z, c);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Scatters of float states.  The node sums are float64 (see the top of this file), but the terms of one
+// run of particles with the same base node are summed as float pairs hi + lo: a product of two floats is
+// exact as a pair (one FMA), a sum of pairs keeps about 48 bits, which is what the read-back grids hold,
+// and the float32 pipe has 64 times the rate of the float64 one.  A warp groups its 32 particles by base
+// node and walks them with its lanes as stencil nodes (warp_kernels.cuh); a run's sums reach the grid as
+// one float64 add per node and component.
+struct Pair {
+  float hi, lo;
+};
+// a + b, exactly (Knuth)
+__device__ __forceinline__ Pair pair_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
+__device__ __forceinline__ Pair pair_prod(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return {p, __fmaf_rn(a, b, -p)};
+}
+// (a.hi + a.lo)(b.hi + b.lo) without the product of the low parts
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+  Pair p = pair_prod(a.hi, b.hi);
+  p.lo = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo));
+  return p;
+}
+__device__ __forceinline__ void pair_add(Pair& s, Pair t) {
+  const Pair u = pair_sum(s.hi, t.hi);
+  const float lo = __fadd_rn(u.lo, __fadd_rn(s.lo, t.lo));
+  s.hi = __fadd_rn(u.hi, lo);
+  s.lo = __fsub_rn(lo, __fsub_rn(s.hi, u.hi));
+}
+
+// Records: kReverse false (forward P2G): [m, v (3), A (9), fx (3)], a node gets w (m v + A dpos) and w m;
+// true (reverse G2P): [vb (3), Cb (9), fx (3)], a node gets w (vb + c4 Cb r).  The factors are formed as in
+// the float64 kernels below: A dpos, c4 Cb r and (reverse) w in float, the products and sums beyond.
+template <bool kReverse>
+__device__ __forceinline__ void adj_scatter(WarpRecs<3, float>& wr, const float (&rec)[16], int node,
+                                            const RunLane<3, float>& ln, const KParams<float>& kp,
+                                            Node4<double>* __restrict__ grid) {
+  const unsigned vmask = __ballot_sync(0xffffffffu, node >= 0);
+  if (vmask == 0u) return;
+  const int nv = warp_group<3, float>(wr, rec, node, vmask);
+  constexpr int NC = kReverse ? 3 : 4, f0 = kReverse ? 12 : 13;
+  const int per = (nv + 2) / 3, l0 = ln.grp * per, l1 = ln.grp < 3 ? min(nv, l0 + per) : 0;
+  const int R = kp.res + 1;
+  const int64_t RR = (int64_t)R * R;
+  Node4<double>* const at = grid + (ln.oa * R + ln.ob);
+  Pair acc[3][NC];
+  int cur = -1;
+  const auto flush = [&]() {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      double* d = &at[cur + i * RR].x;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) atomicAdd(d + c, double(acc[i][c].hi) + double(acc[i][c].lo));
+    }
+  };
+  for (int l = l0; l < l1; ++l) {
+    const int nd = wr.node[l];
+    float rv[16];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 q = *reinterpret_cast<const float4*>(&wr.rec[l][4 * i]);
+      rv[4 * i] = q.x;
+      rv[4 * i + 1] = q.y;
+      rv[4 * i + 2] = q.z;
+      rv[4 * i + 3] = q.w;
+    }
+    if (nd != cur) {
+      if (cur >= 0) flush();
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc[i][c] = {0.f, 0.f};
+      cur = nd;
+    }
+    float wx[3], wy[3], wz[3];
+    bspline(rv[f0], wx);
+    bspline(rv[f0 + 1], wy);
+    bspline(rv[f0 + 2], wz);
+    const float wj = ln.oa == 0 ? wy[0] : ln.oa == 1 ? wy[1] : wy[2];
+    const float wk = ln.ob == 0 ? wz[0] : ln.ob == 1 ? wz[1] : wz[2];
+    if constexpr (kReverse) {
+      const float c4 = 4.f * kp.inv_dx, rj = float(ln.oa) - rv[f0 + 1], rk = float(ln.ob) - rv[f0 + 2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const float wt = wx[i] * wj * wk, ri = float(i) - rv[f0];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float cr = rv[3 + 3 * c] * ri + rv[4 + 3 * c] * rj + rv[5 + 3 * c] * rk;
+          const Pair t = pair_sum(rv[c], c4 * cr);
+          Pair p = pair_prod(wt, t.hi);
+          p.lo = __fmaf_rn(wt, t.lo, p.lo);
+          pair_add(acc[i][c], p);
+        }
+      }
+    } else {
+      const Pair wjk = pair_prod(wj, wk);
+      const float d1 = (float(ln.oa) - rv[f0 + 1]) * kp.dx, d2 = (float(ln.ob) - rv[f0 + 2]) * kp.dx;
+      Pair mv[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) mv[c] = pair_prod(rv[0], rv[1 + c]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        Pair w = pair_prod(wx[i], wjk.hi);
+        w.lo = __fmaf_rn(wx[i], wjk.lo, w.lo);
+        const float d0 = (float(i) - rv[f0]) * kp.dx;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float ad = rv[4 + 3 * c] * d0 + rv[5 + 3 * c] * d1 + rv[6 + 3 * c] * d2;
+          Pair q = pair_sum(mv[c].hi, ad);
+          q.lo = __fadd_rn(q.lo, mv[c].lo);
+          pair_add(acc[i][c], pair_mul(w, q));
+        }
+        Pair wm = pair_prod(w.hi, rv[0]);
+        wm.lo = __fmaf_rn(w.lo, rv[0], wm.lo);
+        pair_add(acc[i][3], wm);
+      }
+    }
+  }
+  if (cur >= 0) flush();
+  __syncwarp();  // the records are rewritten by the warp's next particles
+}
+
+// k_adj_p2g for float states.
+__global__ void __launch_bounds__(kAdjThreads) k_adj_p2g_warp(KParams<float> kp, PView<float> P, uint32_t n,
+                                                              Node4<double>* __restrict__ grid, int32_t* status) {
+  __shared__ WarpRecs<3, float> wrs[kAdjThreads / 32];
+  const RunLane<3, float> ln;
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  float rec[16];
+  int node = -1;
+  if (p < n) {
+    float x[3], v[3], F[9], C[9], fx[3];
+    load_state(P, p, x, v, F, C);
+    int b[3];
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) ok = ok && base_of(x[d], kp.inv_dx, kp.res, b[d], fx[d]);
+    if (!ok) {
+      raise_status(status, FFMPM_STATUS_OOB);
+    } else {
+      node = (int)node_index<3>(kp.res + 1, b);
+      float m, mu, lam, A[9];
+      lame_of(kp, P, p, m, mu, lam);
+      affine_of<3, float>(kp, F, C, m, mu, lam, A, nullptr);
+      rec[0] = m;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        rec[1 + d] = v[d];
+        rec[13 + d] = fx[d];
+      }
+#pragma unroll
+      for (int i = 0; i < 9; ++i) rec[4 + i] = A[i];
+    }
+  }
+  adj_scatter<false>(wrs[threadIdx.x >> 5], rec, node, ln, kp, grid);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -178,8 +344,13 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_gridvel(KParams<double> kp,
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nnodes) return;
   const int R = kp.res + 1;
-  const int I[3] = {(int)(idx / ((int64_t)R * R)), (int)((idx / R) % R), (int)(idx % R)};
+  const uint32_t u = (uint32_t)idx, Ru = (uint32_t)R;  // below 2^31: adj_layout bounds the grid
+  const int I[3] = {(int)(u / (Ru * Ru)), (int)((u / Ru) % Ru), (int)(u % Ru)};
   const Node4<double> g = grid[idx];
+  if (g.x == 0.0 && g.y == 0.0 && g.z == 0.0 && g.w == 0.0) {  // most of the grid: velocity zero, no float64 work
+    store_zero(gvel, idx);
+    return;
+  }
   double vel[3] = {g.x, g.y, g.z};
   grid_node<3, double>(kp, I, vel, g.w);
   store_node(gvel, idx, vel[0], vel[1], vel[2], g.w);
@@ -193,88 +364,111 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_g2p(KParams<T> kp, PView<T>
                                                          const ReadNode<T>* __restrict__ gvel,
                                                          Node4<double>* __restrict__ gadj, int32_t* status) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  T x[3], F[9];
-  load_state<T>(P, p, x, nullptr, F, nullptr);
-  int b[3];
-  T fx[3], w[3][3], dw[3][3];
-  if (!stencil3(kp, x, b, fx, w, dw)) {
+  // float states scatter by whole warps at the end (adj_scatter)
+  constexpr bool kWarp = sizeof(T) == 4;
+  if (!kWarp && p >= n) return;
+  bool ok = p < n;
+  T x[3] = {}, F[9] = {};
+  if (ok) load_state<T>(P, p, x, nullptr, F, nullptr);
+  int b[3] = {};
+  T fx[3] = {}, w[3][3], dw[3][3];
+  if (ok && !stencil3(kp, x, b, fx, w, dw)) {
     raise_status(status, FFMPM_STATUS_OOB);
-    return;
+    ok = false;
   }
-  T xb[3], vb[3], Fb1[9], Cb[9];
+  if (!kWarp && !ok) return;
+  T vb[3] = {}, Cb[9] = {};
+  if (ok) {
+    T xb[3], Fb1[9];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    xb[d] = Ab.x[Ab.at(p, d, 3)];
-    vb[d] = Ab.v[Ab.at(p, d, 3)] + kp.dt * xb[d];  // x' = x + dt v'
-  }
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    Fb1[i] = Ab.F[Ab.at(p, i, 9)];
-    Cb[i] = Ab.C[Ab.at(p, i, 9)];
-  }
-  // C' enters F' = (I + dt C') F: dL/dC' += dt dL/dF' F^T
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      Cb[a * 3 + c] += kp.dt * (Fb1[a * 3 + 0] * F[c * 3 + 0] + Fb1[a * 3 + 1] * F[c * 3 + 1] +
-                                Fb1[a * 3 + 2] * F[c * 3 + 2]);
-  const T c4 = T(4) * kp.inv_dx;
-  // sums over node velocities relative to the centre node's u (as the forward gather): with
-  // dv_i = vg_i - u, sum dW = 0 and sum dW_d (i - fx) = e_d make the u terms of dL/dx cancel, so
-  //   dL/dx_d = inv_dx (sum dW_d (vb.dv_i + c4 dv_i.Cb r_i) - c4 (Cb^T sum W dv_i)_d)
-  T v1[3] = {0, 0, 0}, C1[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, xacc[3] = {0, 0, 0};
-  const int R = kp.res + 1;
-  const ReadNode<T> u = gvel[((int64_t)(b[0] + 1) * R + (b[1] + 1)) * R + (b[2] + 1)];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const T wt = w[i][0] * w[j][1] * w[k][2];
-        const T g0 = dw[i][0] * w[j][1] * w[k][2], g1 = w[i][0] * dw[j][1] * w[k][2],
-                g2 = w[i][0] * w[j][1] * dw[k][2];
-        const T r[3] = {T(i) - fx[0], T(j) - fx[1], T(k) - fx[2]};
-        const int64_t node = ((int64_t)(b[0] + i) * R + (b[1] + j)) * R + (b[2] + k);
-        T vel[4];
-        node_dev(gvel[node], u, vel);
-        T cr[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          v1[a] += wt * vel[a];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) C1[a * 3 + c] += wt * vel[a] * r[c];
-          cr[a] = Cb[a * 3 + 0] * r[0] + Cb[a * 3 + 1] * r[1] + Cb[a * 3 + 2] * r[2];
-        }
-        const T term = vb[0] * vel[0] + vb[1] * vel[1] + vb[2] * vel[2] +
-                       c4 * (vel[0] * cr[0] + vel[1] * cr[1] + vel[2] * cr[2]);
-        xacc[0] += g0 * term;
-        xacc[1] += g1 * term;
-        xacc[2] += g2 * term;
-        const double wd = double(wt);
-        red_add3(&gadj[node], wd * (double(vb[0]) + double(c4 * cr[0])), wd * (double(vb[1]) + double(c4 * cr[1])),
-                 wd * (double(vb[2]) + double(c4 * cr[2])));
-      }
-#pragma unroll
-  for (int i = 0; i < 9; ++i) C1[i] *= c4;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    // v1 holds sum W dv_i here (the u part of v' = u + sum W dv_i cancels, see above)
-    const T ct = Cb[0 * 3 + d] * v1[0] + Cb[1 * 3 + d] * v1[1] + Cb[2 * 3 + d] * v1[2];
-    Ab.x[Ab.at(p, d, 3)] = xb[d] + kp.inv_dx * (xacc[d] - c4 * ct);
-  }
-  // dL/dF = (I + dt C')^T dL/dF'
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      T s = Fb1[a * 3 + c];
-#pragma unroll
-      for (int e = 0; e < 3; ++e) s += kp.dt * C1[e * 3 + a] * Fb1[e * 3 + c];
-      Ab.F[Ab.at(p, a * 3 + c, 9)] = s;
+    for (int d = 0; d < 3; ++d) {
+      xb[d] = Ab.x[Ab.at(p, d, 3)];
+      vb[d] = Ab.v[Ab.at(p, d, 3)] + kp.dt * xb[d];  // x' = x + dt v'
     }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      Fb1[i] = Ab.F[Ab.at(p, i, 9)];
+      Cb[i] = Ab.C[Ab.at(p, i, 9)];
+    }
+    // C' enters F' = (I + dt C') F: dL/dC' += dt dL/dF' F^T
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        Cb[a * 3 + c] += kp.dt * (Fb1[a * 3 + 0] * F[c * 3 + 0] + Fb1[a * 3 + 1] * F[c * 3 + 1] +
+                                  Fb1[a * 3 + 2] * F[c * 3 + 2]);
+    const T c4 = T(4) * kp.inv_dx;
+    // sums over node velocities relative to the centre node's u (as the forward gather): with
+    // dv_i = vg_i - u, sum dW = 0 and sum dW_d (i - fx) = e_d make the u terms of dL/dx cancel, so
+    //   dL/dx_d = inv_dx (sum dW_d (vb.dv_i + c4 dv_i.Cb r_i) - c4 (Cb^T sum W dv_i)_d)
+    T v1[3] = {0, 0, 0}, C1[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, xacc[3] = {0, 0, 0};
+    const int R = kp.res + 1;
+    const ReadNode<T> u = gvel[((int64_t)(b[0] + 1) * R + (b[1] + 1)) * R + (b[2] + 1)];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const T wt = w[i][0] * w[j][1] * w[k][2];
+          const T g0 = dw[i][0] * w[j][1] * w[k][2], g1 = w[i][0] * dw[j][1] * w[k][2],
+                  g2 = w[i][0] * w[j][1] * dw[k][2];
+          const T r[3] = {T(i) - fx[0], T(j) - fx[1], T(k) - fx[2]};
+          const int64_t node = ((int64_t)(b[0] + i) * R + (b[1] + j)) * R + (b[2] + k);
+          T vel[4];
+          node_dev(gvel[node], u, vel);
+          T cr[3];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            v1[a] += wt * vel[a];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) C1[a * 3 + c] += wt * vel[a] * r[c];
+            cr[a] = Cb[a * 3 + 0] * r[0] + Cb[a * 3 + 1] * r[1] + Cb[a * 3 + 2] * r[2];
+          }
+          const T term = vb[0] * vel[0] + vb[1] * vel[1] + vb[2] * vel[2] +
+                         c4 * (vel[0] * cr[0] + vel[1] * cr[1] + vel[2] * cr[2]);
+          xacc[0] += g0 * term;
+          xacc[1] += g1 * term;
+          xacc[2] += g2 * term;
+          if constexpr (!kWarp) {
+            const double wd = double(wt);
+            red_add3(&gadj[node], wd * (double(vb[0]) + double(c4 * cr[0])), wd * (double(vb[1]) + double(c4 * cr[1])),
+                     wd * (double(vb[2]) + double(c4 * cr[2])));
+          }
+        }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) C1[i] *= c4;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      // v1 holds sum W dv_i here (the u part of v' = u + sum W dv_i cancels, see above)
+      const T ct = Cb[0 * 3 + d] * v1[0] + Cb[1 * 3 + d] * v1[1] + Cb[2 * 3 + d] * v1[2];
+      Ab.x[Ab.at(p, d, 3)] = xb[d] + kp.inv_dx * (xacc[d] - c4 * ct);
+    }
+    // dL/dF = (I + dt C')^T dL/dF'
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        T s = Fb1[a * 3 + c];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) s += kp.dt * C1[e * 3 + a] * Fb1[e * 3 + c];
+        Ab.F[Ab.at(p, a * 3 + c, 9)] = s;
+      }
+  }
+  if constexpr (kWarp) {
+    __shared__ WarpRecs<3, float> wrs[kAdjThreads / 32];
+    const RunLane<3, float> ln;
+    float rec[16];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      rec[d] = vb[d];
+      rec[12 + d] = fx[d];
+    }
+#pragma unroll
+    for (int e = 0; e < 9; ++e) rec[3 + e] = Cb[e];
+    rec[15] = 0.f;
+    adj_scatter<true>(wrs[threadIdx.x >> 5], rec, ok ? (int)node_index<3>(kp.res + 1, b) : -1, ln, kp, gadj);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -290,7 +484,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_grid(KParams<double> kp, co
   Node4<double> a = gadj[idx];
   if (a.x == T(0) && a.y == T(0) && a.z == T(0)) return;
   const int R = kp.res + 1;
-  const int I[3] = {(int)(idx / ((int64_t)R * R)), (int)((idx / R) % R), (int)(idx % R)};
+  const uint32_t u = (uint32_t)idx, Ru = (uint32_t)R;  // below 2^31: adj_layout bounds the grid
+  const int I[3] = {(int)(u / (Ru * Ru)), (int)((u / Ru) % Ru), (int)(u % Ru)};
   const Node4<double> g = grid[idx];
   T vb[3] = {a.x, a.y, a.z};
   const T gp[3] = {g.x, g.y, g.z};
@@ -593,7 +788,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj2_gridvel(KParams<double> kp
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nnodes) return;
   const int R = kp.res + 1;
-  const int I[2] = {(int)(idx / R), (int)(idx % R)};
+  const uint32_t u = (uint32_t)idx, Ru = (uint32_t)R;
+  const int I[2] = {(int)(u / Ru), (int)(u % Ru)};
   const Node4<double> g = grid[idx];
   double vel[3] = {g.x, g.y, 0.0};
   grid_node<2, double>(kp, I, vel, g.w);
@@ -686,7 +882,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj2_grid(KParams<double> kp, c
   Node4<double> a = gadj[idx];
   if (a.x == T(0) && a.y == T(0)) return;
   const int R = kp.res + 1;
-  const int I[2] = {(int)(idx / R), (int)(idx % R)};
+  const uint32_t u = (uint32_t)idx, Ru = (uint32_t)R;
+  const int I[2] = {(int)(u / Ru), (int)(u % Ru)};
   const Node4<double> g = grid[idx];
   T vb[2] = {a.x, a.y};
   const T gp[2] = {g.x, g.y};
@@ -887,7 +1084,10 @@ int run_adjoint(const ffmpm_params& p, const AdjLayout& L, const ffmpm_particles
     k_adj2_p2g_rev<T><<<pg, kAdjThreads, 0, s>>>(kp, pv, av, n, gadj, &hdr->status);
     return cudaGetLastError() == cudaSuccess ? FFMPM_OK : FFMPM_ERR_CUDA;
   }
-  k_adj_p2g<T><<<pg, kAdjThreads, 0, s>>>(kp, pv, n, grid, &hdr->status);
+  if constexpr (sizeof(T) == 4)
+    k_adj_p2g_warp<<<pg, kAdjThreads, 0, s>>>(kp, pv, n, grid, &hdr->status);
+  else
+    k_adj_p2g<T><<<pg, kAdjThreads, 0, s>>>(kp, pv, n, grid, &hdr->status);
   using G = ReadNode<T>;
   k_adj_gridvel<G><<<ng, kAdjThreads, 0, s>>>(kd, grid, reinterpret_cast<G*>(gvel), L.nnodes);
   k_adj_g2p<T><<<pg, kAdjThreads, 0, s>>>(kp, pv, av, n, reinterpret_cast<const G*>(gvel), gadj, &hdr->status);

@@ -249,24 +249,13 @@ struct alignas(16) WarpRecs {
   int node[32];
 };
 
+// The grouping alone: `rec` of every lane with a particle into wr, grouped by node.  Returns how many.
 template <int DIM, typename T>
-__device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec_in)[RunRec<DIM>::kPacked], int node,
-                                             const RunLane<DIM, T>& ln, Node4<T>* __restrict__ A, int R) {
+__device__ __forceinline__ int warp_group(WarpRecs<DIM, T>& wr, const T (&rec)[RunRec<DIM>::kPacked], int node,
+                                          unsigned vmask) {
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const bool valid = node >= 0;
-  const unsigned vmask = __ballot_sync(kFull, valid);
-  if (vmask == 0u) return;
-  RunSums<DIM, T> rs;
-  run_velocity<DIM, T>(rec_in, rs.u);
-  T rec[RunRec<DIM>::kPacked];
-#pragma unroll
-  for (int i = 0; i < RunRec<DIM>::kPacked; ++i) rec[i] = rec_in[i];
-#pragma unroll
-  for (int r = 0; r < DIM; ++r) {
-    rs.u[r] = __shfl_sync(kFull, rs.u[r], __ffs(vmask) - 1);
-    rec[1 + r] -= rec[0] * rs.u[r];
-  }
   // slot of the lane's record: the lanes of one base node together, groups in order of first lane
   const unsigned peers = __match_any_sync(kFull, node);
   const unsigned before = peers & lanemask_lt();
@@ -287,12 +276,32 @@ __device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec
     wr.node[slot] = node;
   }
   __syncwarp();
-  const int nv = __popc(vmask);
+  return __popc(vmask);
+}
+
+template <int DIM, typename T>
+__device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec_in)[RunRec<DIM>::kPacked], int node,
+                                             const RunLane<DIM, T>& ln, Node4<T>* __restrict__ A, int R) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const unsigned vmask = __ballot_sync(kFull, node >= 0);
+  if (vmask == 0u) return;
+  RunSums<DIM, T> rs;
+  run_velocity<DIM, T>(rec_in, rs.u);
+  T rec[RunRec<DIM>::kPacked];
+#pragma unroll
+  for (int i = 0; i < RunRec<DIM>::kPacked; ++i) rec[i] = rec_in[i];
+#pragma unroll
+  for (int r = 0; r < DIM; ++r) {
+    rs.u[r] = __shfl_sync(kFull, rs.u[r], __ffs(vmask) - 1);
+    rec[1 + r] -= rec[0] * rs.u[r];
+  }
+  const int nv = warp_group<DIM, T>(wr, rec, node, vmask);
   const int per = (nv + 2) / 3;
   const int l0 = ln.grp * per;
   const int64_t RR = DIM == 3 ? (int64_t)R * R : 0;
   Node4<T>* const Al = A + (ln.oa * R + ln.ob);
-  run_sums<DIM, T, RunRec<DIM>::kSmem, false, false>(rs, &wr.rec[0][0], wr.node, l0, ln.grp < 3 ? min(nv, l0 + per) : 0, ln, Al, RR);
+  run_sums<DIM, T, RunRec<DIM>::kSmem, false, false>(rs, &wr.rec[0][0], wr.node, l0,
+                                                     ln.grp < 3 ? min(nv, l0 + per) : 0, ln, Al, RR);
   run_end<DIM, T>(rs, ln, Al, RR);
   __syncwarp();  // the records are rewritten by the warp's next particles
 }
