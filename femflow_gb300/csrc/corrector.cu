@@ -1,11 +1,15 @@
 // Learned-corrector G2P: the 3D G2P of a coarse substep (three_d/g2p.py:9-59) fused with a
 // per-particle MLP that corrects its result, run on the 5th-generation tensor cores.
 //
-// One CTA = 128 threads = 128 particles per tile (persistent over tiles); thread t owns particle
-// (tile * 128 + t) and TMEM lane t, i.e. row t of every MLP layer.  Per tile:
-//   1. each thread gathers its 27 stencil nodes from the updated grid, forms v', C', F' and x' as the
-//      plain G2P does (node velocities taken relative to the stencil's centre node u), and writes
-//      its 128 bf16 features into row t of the K-major input tile in shared memory:
+// A CTA of 512 threads is four warpgroups, each on a tile of 128 particles of its own (persistent over
+// tiles; thread t of a group owns particle tile * 128 + t and TMEM lane t, i.e. row t of every MLP
+// layer); they share the weights and hide one another's latencies.  Per tile:
+//   1. the 27 node velocities of every particle come to shared memory a plane of nine nodes at a time:
+//      a warp takes its 32 particles one after another, its lanes on the 27 floats of a plane (three runs
+//      of nine), so that one asynchronous load instruction touches a few lines where a load per thread
+//      and float touches 32.  Each thread then forms v', C', F' and x' as the plain G2P does (node
+//      velocities taken relative to the stencil's centre node u) and its bf16 features in row t of the
+//      K-major input tile, eight to a store:
 //        [0, 9)   F' - I            [9, 18)  C' dt            [18, 21) (v' - u) dt / dx
 //        [21,102) (v_i - u) dt / dx for the 27 nodes i
 //        [102,104) mu k, lam k      [104,113) PF k (the stress of this step's P2G)      [113,128) 0
@@ -15,6 +19,9 @@
 //      TMEM; after each layer every thread reads its own row back (tcgen05.ld), adds the bias,
 //      applies GELU and writes the bf16 row of the next layer's operand;
 //   3. outputs y[0,12) times the output scale: F' += y[0,9), v' += y[9,12) dx / dt, x' += dt * that.
+// 1,048,576 particles of a random order on 128^3 (GB300): 337 us, from 580 with one tile of 128 threads a CTA,
+// loads and feature stores one float and one bf16 at a time and erff; bound by instruction issue (GELU of
+// 192 units a particle) and the gathers' latency.
 // Weights (bf16, K-major) and biases stay in shared memory for the whole launch.  Modes: apply the
 // network, export the features (no network), or both off (the plain coarse G2P through the same
 // arithmetic).  Every mbarrier wait is bounded.
@@ -37,22 +44,57 @@ constexpr int kOutPad = 16;
 constexpr int kOut = FFMPM_MLP_OUT;  // 12
 constexpr uint32_t kSboIn = (kIn / 8) * 128;
 constexpr uint32_t kSboHid = (kHid / 8) * 128;
-constexpr int kThreadsC = 128;
-constexpr uint32_t kTmemCols = 128;  // [0, 64): hidden layers, [64, 80): output layer
+constexpr int kGroups = 4;                  // warpgroups (tiles in flight) per CTA
+constexpr int kThreadsC = 128 * kGroups;
+constexpr uint32_t kTmemCols = 128;         // per group: [0, 64) hidden layers, [64, 80) output layer
+constexpr int kPlane = 27;                  // floats of a plane of nine nodes
 
 struct SmemLayout {
   static constexpr size_t w1 = 0;
   static constexpr size_t w2 = w1 + size_t(kHid) * kIn * 2;
   static constexpr size_t w3 = w2 + size_t(kHid) * kHid * 2;
   static constexpr size_t w4 = w3 + size_t(kHid) * kHid * 2;
-  static constexpr size_t x = w4 + size_t(kOutPad) * kHid * 2;
-  static constexpr size_t h = x + size_t(128) * kIn * 2;
-  static constexpr size_t f = h + size_t(128) * kHid * 2;  // floats: b1 b2 b3 b4 in_scale out_scale
+  static constexpr size_t f = w4 + size_t(kOutPad) * kHid * 2;  // floats: b1 b2 b3 b4 in_scale out_scale
   static constexpr int nf = 3 * kHid + kOutPad + kIn + kOutPad;
-  static constexpr size_t total = f + sizeof(float) * nf;
+  static constexpr size_t group = f + sizeof(float) * nf;  // per group: input tile, then a plane of velocities
+  static constexpr size_t x_bytes = size_t(128) * kIn * 2;  // the hidden layers' tile lies over the input tile
+  static constexpr size_t group_bytes = x_bytes + size_t(128) * kPlane * 4;
+  static constexpr size_t total = group + kGroups * group_bytes;
 };
+static_assert(SmemLayout::group % 128 == 0 && SmemLayout::group_bytes % 128 == 0, "aligned tiles");
+static_assert(SmemLayout::total <= 227 * 1024 - 1024, "one CTA per SM");
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
+// GELU(z) = z Phi(z), with Phi(-a) = 2^p(a) for a = |z| and GELU(z) = max(z, 0) - a Phi(-a).  p: degree-10
+// polynomial fitted to log2 of the normal distribution function on [0, 6] (reweighted least squares at
+// Chebyshev points, largest error 3.6e-7; beyond 6 the value at 6, below 1e-8).  In float over [-8, 8]: largest
+// absolute error 2.4e-7, rms 5.2e-8, and 1.2e-6 relative for |z| < 4; 0.5 z (1 + erff(z / sqrt 2)) has
+// 4.5e-7, 6.8e-8 and (where 1 + erf cancels) 4.6e-4.  Two at a time: the polynomial runs on packed FMAs.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ void gelu2(float z0, float z1, float& g0, float& g1) {
+  constexpr float kP[11] = {-0.999999642f, -1.15111935f, -0.459117204f, -0.0527117103f, 0.0073000202f, -0.000260737259f, -0.000164237936f, 4.52711574e-05f, -5.93813365e-06f, 4.14644262e-07f, -1.23162778e-08f};
+  const float a0 = fabsf(z0), a1 = fabsf(z1);
+  const uint64_t a = pack2(fminf(a0, 6.f), fminf(a1, 6.f));
+  uint64_t p = pack2(kP[10], kP[10]);
+#pragma unroll
+  for (int i = 9; i >= 0; --i) p = fma2(p, a, pack2(kP[i], kP[i]));
+  float p0, p1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(p0), "=f"(p1) : "l"(p));
+  g0 = fmaf(-a0, exp2f(p0), fmaxf(z0, 0.f));
+  g1 = fmaf(-a1, exp2f(p1), fmaxf(z1, 0.f));
+}
+
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+  return uint32_t(tc::bf16_bits(a)) | (uint32_t(tc::bf16_bits(b)) << 16);
+}
 
 // Copy a bf16 row-major [rows][k] matrix into the K-major core-matrix layout.
 __device__ __forceinline__ void stage_kmajor(unsigned char* dst, const uint16_t* src, int rows, int k, uint32_t sbo) {
@@ -64,15 +106,15 @@ __device__ __forceinline__ void stage_kmajor(unsigned char* dst, const uint16_t*
   }
 }
 
-// Two consecutive features (k even) of row r as one 32-bit shared store.
-__device__ __forceinline__ void put2(unsigned char* tile, int r, int k, uint32_t sbo, float a, float b) {
-  const uint32_t w = uint32_t(tc::bf16_bits(a)) | (uint32_t(tc::bf16_bits(b)) << 16);
-  *reinterpret_cast<uint32_t*>(tile + tc::kmajor_offset(r, k, sbo)) = w;
+// Eight consecutive features (from 8 c on) of row r as one 16-byte store, scaled.
+__device__ __forceinline__ void put8(unsigned char* tile, int r, int c, const float (&f)[8], const float* s_in) {
+  const float4 s0 = *reinterpret_cast<const float4*>(s_in + 8 * c), s1 = *reinterpret_cast<const float4*>(s_in + 8 * c + 4);
+  *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(r, 8 * c, kSboIn)) =
+      make_uint4(bf16x2(f[0] * s0.x, f[1] * s0.y), bf16x2(f[2] * s0.z, f[3] * s0.w), bf16x2(f[4] * s1.x, f[5] * s1.y),
+                 bf16x2(f[6] * s1.z, f[7] * s1.w));
 }
 
-__device__ __forceinline__ void put1(unsigned char* tile, int r, int k, uint32_t sbo, float a) {
-  *reinterpret_cast<uint16_t*>(tile + tc::kmajor_offset(r, k, sbo)) = tc::bf16_bits(a);
-}
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
 
 // Order-preserving float -> int key (for atomicMin / atomicMax on signed floats).
 __device__ __forceinline__ int float_key(float f) {
@@ -81,164 +123,248 @@ __device__ __forceinline__ int float_key(float f) {
 }
 
 template <bool kApply, bool kExport>
-__global__ void __launch_bounds__(kThreadsC) k_corrector(KParams<float> kp, const float* __restrict__ gv,
-                                                         PView<float> P, uint32_t n, ffmpm_mlp net,
-                                                         uint16_t* __restrict__ feat_out, int* __restrict__ det_keys,
-                                                         int32_t* status) {
+__global__ void __launch_bounds__(kThreadsC, 1) k_corrector(KParams<float> kp, const float* __restrict__ gv,
+                                                            PView<float> P, uint32_t n, ffmpm_mlp net,
+                                                            uint16_t* __restrict__ feat_out,
+                                                            int* __restrict__ det_keys, int32_t* status) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* sW1 = smem + SmemLayout::w1;
-  unsigned char* sW2 = smem + SmemLayout::w2;
-  unsigned char* sW3 = smem + SmemLayout::w3;
-  unsigned char* sW4 = smem + SmemLayout::w4;
-  unsigned char* sX = smem + SmemLayout::x;
-  unsigned char* sH = smem + SmemLayout::h;
-  float* sf = reinterpret_cast<float*>(smem + SmemLayout::f);
-  float* sb1 = sf;
-  float* sb2 = sb1 + kHid;
-  float* sb3 = sb2 + kHid;
-  float* sb4 = sb3 + kHid;
-  float* s_in = sb4 + kOutPad;
-  float* s_out = s_in + kIn;
-  __shared__ uint64_t bar;
+  float* const sbias = reinterpret_cast<float*>(smem + SmemLayout::f);  // b1, b2, b3
+  float* const sb4 = sbias + 3 * kHid;
+  float* const s_in = sb4 + kOutPad;
+  float* const s_out = s_in + kIn;
+  __shared__ uint64_t bars[kGroups];
   __shared__ uint32_t tmem_base;
-  __shared__ int s_fail;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  __shared__ int s_fail[kGroups];
+  const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31;
+  unsigned char* const sX = smem + SmemLayout::group + grp * SmemLayout::group_bytes;
+  float* const sV = reinterpret_cast<float*>(sX + SmemLayout::x_bytes);  // [128][kPlane]
+  float* const warpV = sV + (tid & ~31) * kPlane;
 
-  for (int i = tid; i < kIn; i += kThreadsC) s_in[i] = net.in_scale ? net.in_scale[i] : 1.f;
+  for (int i = threadIdx.x; i < kIn; i += kThreadsC) s_in[i] = net.in_scale ? net.in_scale[i] : 1.f;
   if (kApply) {
-    stage_kmajor(sW1, net.W1, kHid, kIn, kSboIn);
-    stage_kmajor(sW2, net.W2, kHid, kHid, kSboHid);
-    stage_kmajor(sW3, net.W3, kHid, kHid, kSboHid);
-    stage_kmajor(sW4, net.W4, kOutPad, kHid, kSboHid);
-    for (int i = tid; i < kHid; i += kThreadsC) {
-      sb1[i] = net.b1[i];
-      sb2[i] = net.b2[i];
-      sb3[i] = net.b3[i];
+    stage_kmajor(smem + SmemLayout::w1, net.W1, kHid, kIn, kSboIn);
+    stage_kmajor(smem + SmemLayout::w2, net.W2, kHid, kHid, kSboHid);
+    stage_kmajor(smem + SmemLayout::w3, net.W3, kHid, kHid, kSboHid);
+    stage_kmajor(smem + SmemLayout::w4, net.W4, kOutPad, kHid, kSboHid);
+    for (int i = threadIdx.x; i < kHid; i += kThreadsC) {
+      sbias[i] = net.b1[i];
+      sbias[kHid + i] = net.b2[i];
+      sbias[2 * kHid + i] = net.b3[i];
     }
-    for (int i = tid; i < kOutPad; i += kThreadsC) {
+    for (int i = threadIdx.x; i < kOutPad; i += kThreadsC) {
       sb4[i] = net.b4[i];
       s_out[i] = net.out_scale[i];
     }
-    if (warp == 0) tc::tmem_alloc(&tmem_base, kTmemCols);
+    if (threadIdx.x < 32) tc::tmem_alloc(&tmem_base, kGroups * kTmemCols);
+    fence_proxy_async_shared();
   }
-  if (tid == 0) {
-    mbar_init(&bar, 1);
+  if (threadIdx.x < kGroups) {
+    mbar_init(&bars[threadIdx.x], 1);
     fence_barrier_init();
-    s_fail = 0;
+    s_fail[threadIdx.x] = 0;
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = kApply ? tmem_base : 0u;
-  const uint32_t lane_base = 32u * warp;
+  const uint32_t tmem = (kApply ? tmem_base : 0u) + grp * kTmemCols;
+  uint64_t* const bar = &bars[grp];
+  const uint32_t lane_base = 32u * (tid >> 5);
   uint32_t phase = 0;
   const float dt = kp.dt, inv_dx = kp.inv_dx;
   const float vs = dt * inv_dx;  // velocity -> cells per step
+  const int R = kp.res + 1;
+  const int64_t RR = (int64_t)R * R;
   float dmin = 3.4e38f, dmax = -3.4e38f;
 
-  for (uint32_t tile = blockIdx.x; tile * 128u < n; tile += gridDim.x) {
-    const uint32_t p = tile * 128u + tid;
+  // neighbouring groups of a CTA take tiles a grid apart, so that few tiles spread over the SMs
+  for (int64_t tile = blockIdx.x + (int64_t)gridDim.x * grp; tile * 128 < n; tile += (int64_t)gridDim.x * kGroups) {
+    const uint32_t p = (uint32_t)(tile * 128 + tid);
     bool valid = p < n;
     float xo[3], Fo[9], Co[9], vo[3];
+    float x[3], fx[3], w[3][3];
+    int node = -1;
     if (valid) {
-      float x[3], F[9], fx[3], w[3][3];  // pre-step state and stencil
       int b[3];
+      bool ok = true;
 #pragma unroll
       for (int d = 0; d < 3; ++d) x[d] = P.x[P.at(p, d, 3)];
 #pragma unroll
-      for (int i = 0; i < 9; ++i) F[i] = P.F[P.at(p, i, 9)];
-      bool ok = true;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        ok = ok && base_of(x[d], inv_dx, kp.res, b[d], fx[d]);
-        float ww[3];
-        bspline(fx[d], ww);
-        w[0][d] = ww[0];
-        w[1][d] = ww[1];
-        w[2][d] = ww[2];
-      }
+      for (int d = 0; d < 3; ++d) ok = ok && base_of(x[d], inv_dx, kp.res, b[d], fx[d]);
       if (!ok) {
         raise_status(status, FFMPM_STATUS_OOB);
         valid = false;
       } else {
-        const int R = kp.res + 1;
-        const size_t cn = ((size_t)(b[0] + 1) * R + (b[1] + 1)) * R + (b[2] + 1);
-        const float u[3] = {gv[3 * cn + 0], gv[3 * cn + 1], gv[3 * cn + 2]};
-        float v[3] = {0.f, 0.f, 0.f}, C[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        int node = 0;
+        node = (int)node_index<3>(R, b);
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j)
-#pragma unroll
-            for (int k = 0; k < 3; ++k, ++node) {
-              const float wt = w[i][0] * w[j][1] * w[k][2];
-              const size_t gi = ((size_t)(b[0] + i) * R + (b[1] + j)) * R + (b[2] + k);
-              const float d0 = gv[3 * gi + 0] - u[0], d1 = gv[3 * gi + 1] - u[1], d2 = gv[3 * gi + 2] - u[2];
-              const float r0 = float(i) - fx[0], r1 = float(j) - fx[1], r2 = float(k) - fx[2];
-              v[0] += wt * d0;
-              v[1] += wt * d1;
-              v[2] += wt * d2;
-              C[0] += wt * d0 * r0; C[1] += wt * d0 * r1; C[2] += wt * d0 * r2;
-              C[3] += wt * d1 * r0; C[4] += wt * d1 * r1; C[5] += wt * d1 * r2;
-              C[6] += wt * d2 * r0; C[7] += wt * d2 * r1; C[8] += wt * d2 * r2;
-              const int f0 = 21 + 3 * node;  // features of node `node`
-              put1(sX, tid, f0, kSboIn, d0 * vs * s_in[f0]);
-              put1(sX, tid, f0 + 1, kSboIn, d1 * vs * s_in[f0 + 1]);
-              put1(sX, tid, f0 + 2, kSboIn, d2 * vs * s_in[f0 + 2]);
-            }
-        const float c4 = 4.f * inv_dx;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) Co[i] = C[i] * c4;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) vo[d] = u[d] + v[d];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            Fo[r * 3 + c] = F[r * 3 + c] + dt * (Co[r * 3 + 0] * F[0 * 3 + c] + Co[r * 3 + 1] * F[1 * 3 + c] +
-                                                 Co[r * 3 + 2] * F[2 * 3 + c]);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) xo[d] = x[d] + dt * vo[d];
-        // features 0..20, then zero padding 102..127
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-          put1(sX, tid, i, kSboIn, (Fo[i] - (i % 4 == 0 ? 1.f : 0.f)) * s_in[i]);
-          put1(sX, tid, 9 + i, kSboIn, Co[i] * dt * s_in[9 + i]);
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) put1(sX, tid, 18 + d, kSboIn, v[d] * vs * s_in[18 + d]);
-        // material and stress features 102..112 (from the pre-step F, as the P2G of this step)
-        {
-          float m_, mu_, lam_;
-          lame_of(kp, P, p, m_, mu_, lam_);
-          const float kk = dt * dt * inv_dx * inv_dx * kp.volume / m_;
-          float FmR[9];
-          if (!f_minus_r_small_strain3(F, FmR)) {
-            float Rr[9];
-            polar3<float>(F, Rr, nullptr);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) FmR[i] = F[i] - Rr[i];
-          }
-          const float J = det3(F);
-          const float sc = lam_ * (J - 1.f) * J;
-          put1(sX, tid, 102, kSboIn, mu_ * kk * s_in[102]);
-          put1(sX, tid, 103, kSboIn, lam_ * kk * s_in[103]);
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              float pf = (a == c || kp.model != FFMPM_MODEL_FIXED_COROTATED) ? sc : 0.f;
-#pragma unroll
-              for (int e = 0; e < 3; ++e) pf += 2.f * mu_ * FmR[a * 3 + e] * F[c * 3 + e];
-              put1(sX, tid, 104 + a * 3 + c, kSboIn, pf * kk * s_in[104 + a * 3 + c]);
-            }
-          for (int k = 113; k < 120; ++k) put1(sX, tid, k, kSboIn, 0.f);
-          *reinterpret_cast<uint4*>(sX + tc::kmajor_offset(tid, 120, kSboIn)) = make_uint4(0u, 0u, 0u, 0u);
+        for (int d = 0; d < 3; ++d) {
+          float ww[3];
+          bspline(fx[d], ww);
+          w[0][d] = ww[0];
+          w[1][d] = ww[1];
+          w[2][d] = ww[2];
         }
       }
     }
-    if (!valid) {
+    float u[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f}, C[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (valid) {
+      const float* c = gv + 3 * (node + RR + R + 1);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) u[d] = c[d];
+    }
+    float wzd[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) wzd[k] = valid ? w[k][2] * (float(k) - fx[2]) : 0.f;
+    float keep[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // features of a chunk of eight that a later plane completes
+    float first[3] = {0.f, 0.f, 0.f};                 // features 21..23, for the chunk 16..23
+    const int sj = lane / 9;  // the lane's run of nine floats (27 lanes) and its place in it
+    const int64_t soff = (int64_t)3 * sj * R + (lane - 9 * sj);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      __syncwarp();  // the previous plane (or tile) has been read
+      for (int l = 0; l < 32; ++l) {
+        const int nb = __shfl_sync(0xffffffffu, node, l);
+        if (nb >= 0 && lane < kPlane)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(warpV + l * kPlane + lane)),
+                       "l"(gv + 3 * (nb + i * RR) + soff)
+                       : "memory");
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      if (valid) {
+        const float* g = sV + tid * kPlane;
+        float f[kPlane];
+        float t0[3] = {0.f, 0.f, 0.f}, t1[3] = {0.f, 0.f, 0.f}, t2[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          float sa[3] = {0.f, 0.f, 0.f}, sb[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+              const float d = g[9 * j + 3 * k + r] - u[r];
+              sa[r] += w[k][2] * d;
+              sb[r] += wzd[k] * d;
+              f[9 * j + 3 * k + r] = d * vs;
+            }
+          const float wy = w[j][1], wyd = wy * (float(j) - fx[1]);
+#pragma unroll
+          for (int r = 0; r < 3; ++r) {
+            t0[r] += wy * sa[r];
+            t1[r] += wyd * sa[r];
+            t2[r] += wy * sb[r];
+          }
+        }
+        const float wx = w[i][0], wxd = wx * (float(i) - fx[0]);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          v[r] += wx * t0[r];
+          C[r * 3 + 0] += wxd * t0[r];
+          C[r * 3 + 1] += wx * t1[r];
+          C[r * 3 + 2] += wx * t2[r];
+        }
+        // features 21 + 27 i ...: whole chunks of eight go out, the ends wait for their neighbours
+        float q[8];
+        if (i == 0) {
+#pragma unroll
+          for (int e = 0; e < 3; ++e) first[e] = f[e];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) q[e] = f[3 + 8 * c + e];
+            put8(sX, tid, 3 + c, q, s_in);
+          }
+        } else if (i == 1) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) q[e] = f[8 * c + e];
+            put8(sX, tid, 6 + c, q, s_in);
+          }
+#pragma unroll
+          for (int e = 0; e < 3; ++e) keep[e] = f[24 + e];
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) q[e] = e < 3 ? keep[e] : f[e - 3];
+          put8(sX, tid, 9, q, s_in);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) q[e] = f[5 + 8 * c + e];
+            put8(sX, tid, 10 + c, q, s_in);
+          }
+#pragma unroll
+          for (int e = 0; e < 6; ++e) keep[e] = f[21 + e];
+        }
+      }
+    }
+    if (valid) {
+      float F[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) F[i] = P.F[P.at(p, i, 9)];
+      const float c4 = 4.f * inv_dx;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) Co[i] = C[i] * c4;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) vo[d] = u[d] + v[d];
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          Fo[r * 3 + c] = F[r * 3 + c] + dt * (Co[r * 3 + 0] * F[0 * 3 + c] + Co[r * 3 + 1] * F[1 * 3 + c] +
+                                               Co[r * 3 + 2] * F[2 * 3 + c]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) xo[d] = x[d] + dt * vo[d];
+      // material and stress features 102..112 (from the pre-step F, as the P2G of this step)
+      float m_, mu_, lam_, FmR[9];
+      lame_of(kp, P, p, m_, mu_, lam_);
+      const float kk = dt * dt * inv_dx * inv_dx * kp.volume / m_;
+      if (!f_minus_r_small_strain3(F, FmR)) {
+        float Rr[9];
+        polar3<float>(F, Rr, nullptr);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) FmR[i] = F[i] - Rr[i];
+      }
+      const float J = det3(F);
+      const float sc = lam_ * (J - 1.f) * J;
+      float pf[9];
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          float s = (a == c || kp.model != FFMPM_MODEL_FIXED_COROTATED) ? sc : 0.f;
+#pragma unroll
+          for (int e = 0; e < 3; ++e) s += 2.f * mu_ * FmR[a * 3 + e] * F[c * 3 + e];
+          pf[a * 3 + c] = s * kk;
+        }
+      float h[24];  // features 0..23
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        h[i] = Fo[i] - (i % 4 == 0 ? 1.f : 0.f);
+        h[9 + i] = Co[i] * dt;
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        h[18 + d] = v[d] * vs;
+        h[21 + d] = first[d];
+      }
+      float q[8];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[e] = h[8 * c + e];
+        put8(sX, tid, c, q, s_in);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[e] = e < 6 ? keep[e] : e == 6 ? mu_ * kk : lam_ * kk;
+      put8(sX, tid, 12, q, s_in);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[e] = pf[e];
+      put8(sX, tid, 13, q, s_in);
+      // 112 is the last feature; the padding is zero whatever its scales
+      *reinterpret_cast<uint4*>(sX + tc::kmajor_offset(tid, 112, kSboIn)) =
+          make_uint4(bf16x2(pf[8] * s_in[112], 0.f), 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(sX + tc::kmajor_offset(tid, 120, kSboIn)) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
 #pragma unroll
       for (int k = 0; k < kIn; k += 8)
         *reinterpret_cast<uint4*>(sX + tc::kmajor_offset(tid, k, kSboIn)) = make_uint4(0u, 0u, 0u, 0u);
@@ -254,41 +380,52 @@ __global__ void __launch_bounds__(kThreadsC) k_corrector(KParams<float> kp, cons
       for (int layer = 0; layer < 4; ++layer) {
         fence_proxy_async_shared();
         tc::fence_before_sync();
-        __syncthreads();
+        group_sync(grp);
         tc::fence_after_sync();
         if (tid == 0) {
-          const unsigned char* A = layer == 0 ? sX : sH;
-          const unsigned char* B = layer == 0 ? sW1 : layer == 1 ? sW2 : layer == 2 ? sW3 : sW4;
+          // the hidden layers' tile lies where the input tile was: an MMA has read it before it is rewritten
+          const unsigned char* B = smem + (layer == 0   ? SmemLayout::w1
+                                           : layer == 1 ? SmemLayout::w2
+                                           : layer == 2 ? SmemLayout::w3
+                                                        : SmemLayout::w4);
           const int ksteps = (layer == 0 ? kIn : kHid) / 16;
           const uint32_t sbo = layer == 0 ? kSboIn : kSboHid;
           const uint32_t idesc = layer == 3 ? tc::idesc_bf16_f32(128, kOutPad) : tc::idesc_bf16_f32(128, kHid);
           const uint32_t d = tmem + (layer == 3 ? 64u : 0u);
-          const uint32_t a0 = tc::smem_addr(A), b0 = tc::smem_addr(B);
+          const uint32_t a0 = tc::smem_addr(sX), b0 = tc::smem_addr(B);
           for (int s = 0; s < ksteps; ++s)
             tc::mma_bf16(d, tc::make_desc(a0 + 256u * s, tc::kLBO, sbo), tc::make_desc(b0 + 256u * s, tc::kLBO, sbo),
                          idesc, s > 0);
-          tc::commit(&bar);
+          tc::commit(bar);
         }
-        if (!mbar_wait(&bar, phase)) s_fail = 1;
+        if (!mbar_wait(bar, phase)) s_fail[grp] = 1;
         phase ^= 1u;
         tc::fence_after_sync();
-        __syncthreads();
-        if (s_fail) break;
+        group_sync(grp);
+        if (s_fail[grp]) break;
         if (layer < 3) {
-          const float* bias = layer == 0 ? sb1 : layer == 1 ? sb2 : sb3;
+          const float* bias = sbias + kHid * layer;
 #pragma unroll 1
           for (int c0 = 0; c0 < kHid; c0 += 16) {
             float a[16];
             tc::tmem_ld16(tc::taddr_of(tmem, lane_base, c0), a);
+            uint32_t h[8];
 #pragma unroll
-            for (int j = 0; j < 16; j += 2)
-              put2(sH, tid, c0 + j, kSboHid, gelu(a[j] + bias[c0 + j]), gelu(a[j + 1] + bias[c0 + j + 1]));
+            for (int j = 0; j < 8; ++j) {
+              float g0, g1;
+              gelu2(a[2 * j] + bias[c0 + 2 * j], a[2 * j + 1] + bias[c0 + 2 * j + 1], g0, g1);
+              h[j] = bf16x2(g0, g1);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              *reinterpret_cast<uint4*>(sX + tc::kmajor_offset(tid, c0 + 8 * j, kSboHid)) =
+                  make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
           }
         } else {
           tc::tmem_ld16(tc::taddr_of(tmem, lane_base, 64u), y);
         }
       }
-      if (s_fail) break;
+      if (s_fail[grp]) break;
       if (valid) {
 #pragma unroll
         for (int i = 0; i < 9; ++i) Fo[i] += (y[i] + sb4[i]) * s_out[i];
@@ -316,14 +453,14 @@ __global__ void __launch_bounds__(kThreadsC) k_corrector(KParams<float> kp, cons
       dmin = fminf(dmin, J);
       dmax = fmaxf(dmax, J);
     }
-    // the next tile rewrites sX / sH: every thread is past this tile's MMAs and reads
-    __syncthreads();
+    // the next tile rewrites the group's tile: every thread is past this tile's MMAs and reads
+    group_sync(grp);
   }
-  if (s_fail && tid == 0) {
+  if (s_fail[grp] && tid == 0) {
     raise_status(status, FFMPM_STATUS_TIMEOUT);
     // the MMAs of the last commit may still be running: wait for them once more (bounded) before
     // their tensor memory is freed
-    mbar_wait(&bar, phase ^ 1u);
+    mbar_wait(bar, phase ^ 1u);
   }
   if (det_keys) {
 #pragma unroll
@@ -331,7 +468,7 @@ __global__ void __launch_bounds__(kThreadsC) k_corrector(KParams<float> kp, cons
       dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
       dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
     }
-    if ((tid & 31) == 0 && dmin <= dmax) {
+    if (lane == 0 && dmin <= dmax) {
       atomicMin(&det_keys[0], float_key(dmin));
       atomicMax(&det_keys[1], float_key(dmax));
     }
@@ -339,7 +476,7 @@ __global__ void __launch_bounds__(kThreadsC) k_corrector(KParams<float> kp, cons
   if (kApply) {
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_free(tmem, kTmemCols);
+    if (threadIdx.x < 32) tc::tmem_free(tmem_base, kGroups * kTmemCols);
   }
 }
 
@@ -351,24 +488,10 @@ int launch_corrector(const ffmpm_params& p, const ffmpm_grid& g, ffmpm_particles
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     attr = true;
   }
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreadsC, smem) != cudaSuccess) {
-    cudaGetLastError();
-    per_sm = 1;
-  }
-  {
-    // CTAs per SM that the shared memory holds (each CTA also takes 1 KB reserved by the system)
-    int dev = 0, smem_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    const int by_smem = smem_sm / (int)(smem + 2048);
-    per_sm = std::max(per_sm, std::min(by_smem, 4));
-  }
   const int64_t tiles = (Pp.n + 127) / 128;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, int64_t(sm_count()) * std::max(1, per_sm)));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count()));
   ffmpm_mlp nn{};
   if (net) nn = *net;
   kern<<<grid, kThreadsC, smem, s>>>(kparams<float>(p), static_cast<const float*>(g.velocity), pview<float>(Pp),
