@@ -166,7 +166,13 @@ def load(build_if_missing: bool = False):
         return lib
 
 
+_entries: dict = {}  # entry points looked up so far
+
+
 def call(name: str, *args) -> None:
-    rc = getattr(load(), name)(*args)
+    fn = _entries.get(name)
+    if fn is None:
+        fn = _entries[name] = getattr(load(), name)
+    rc = fn(*args)
     if rc != OK:
         raise RuntimeError(f"{name} failed: {ERRORS.get(rc, rc)}")

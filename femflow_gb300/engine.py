@@ -18,7 +18,10 @@ _WS_CACHE: dict = {}
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = device.index if isinstance(device, torch.device) else None
+    if index is None or not torch.cuda.is_initialized():
+        return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(index)  # the same stream without its Python object
 
 
 def _require_cuda():
@@ -205,6 +208,15 @@ def stage(arrays, device=None, dtype=None) -> Staged:
             t = t.contiguous()
         dev.append(t)
     return Staged(dev, host)
+
+
+def on_device(dtype, arrays) -> bool:
+    """True when every array is a contiguous CUDA tensor of ``dtype`` (or None): nothing to stage, to
+    check or to write back."""
+    for a in arrays:
+        if a is not None and not (isinstance(a, torch.Tensor) and a.is_cuda and a.dtype == dtype and a.is_contiguous()):
+            return False
+    return True
 
 
 def check_tensors(dtype, *tensors):

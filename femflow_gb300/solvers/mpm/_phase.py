@@ -43,6 +43,16 @@ def pinned_host(*arrays) -> bool:
                             and a.dtype == ts[0].dtype for a in ts) and ts[0].dtype in (torch.float32, torch.float64)
 
 
+def staged(arrays, dtype):
+    """The arrays on the GPU, and the Staged that writes host originals back (None when every array is
+    a CUDA tensor already, in which case there is nothing to write back either)."""
+    if E.on_device(dtype, arrays) and any(a is not None for a in arrays):
+        return arrays, None
+    st = E.stage(arrays, dtype=dtype)
+    E.check_tensors(dtype, *st.dev)
+    return st.dev, st
+
+
 _MIRRORS: dict = {}
 
 

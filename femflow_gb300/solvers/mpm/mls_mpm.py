@@ -40,13 +40,12 @@ def solve_mls_mpm_3d(res, inv_dx, hardening, dx, dt, volume, gravity, particles,
                             deterministic=deterministic)
         P.run_host_substep(prm, *host, check=check)
         return
-    st = E.stage([pset.pos, pset.mass, pset.mu_0, pset.lambda_0, v, F, C, Jp], dtype=dtype)
-    x, m, mu, lam, vv, FF, CC, JJ = st.dev
-    E.check_tensors(dtype, x, m, mu, lam, vv, FF, CC, JJ)
+    (x, m, mu, lam, vv, FF, CC, JJ), st = P.staged(host, dtype)
     prm = E.make_params(3, res, dtype, dx, inv_dx, dt, gravity, volume, hardening, model="neo_hookean",
                         deterministic=deterministic)
     ps = E.particles_struct(x, vv, FF, CC, JJ, m, mu, lam)
     P.run("ffmpm_substep", prm, ps.n, x.device, ctypes.byref(prm), ctypes.byref(ps), check=check)
-    st.write_back([0, 4, 5, 6, 7])
+    if st is not None:
+        st.write_back([0, 4, 5, 6, 7])
     if plist is not None:
         pset.write_positions(plist)

@@ -24,43 +24,41 @@ def p2g(inv_dx, hardening, dx, dt, volume, grid_velocity, grid_mass, particles, 
     """
     pset, plist = P.split_particles(particles)
     dtype = P.dtype_of(v, F, grid_velocity)
-    st = E.stage([pset.pos, pset.mass, pset.mu_0, pset.lambda_0, v, F, C, Jp, grid_velocity, grid_mass], dtype=dtype)
-    x, m, mu, lam, vv, FF, CC, JJ, gv, gm = st.dev
-    E.check_tensors(dtype, x, m, mu, lam, vv, FF, CC, JJ, gv, gm)
+    arrays = [pset.pos, pset.mass, pset.mu_0, pset.lambda_0, v, F, C, Jp, grid_velocity, grid_mass]
+    (x, m, mu, lam, vv, FF, CC, JJ, gv, gm), st = P.staged(arrays, dtype)
     res = gv.shape[0] - 1
     prm = E.make_params(3, res, dtype, dx, inv_dx, dt, 0.0, volume, hardening, model=model,
                         deterministic=deterministic)
     ps = E.particles_struct(x, vv, FF, CC, JJ, m, mu, lam)
     g = E.grid_struct(gv, gm)
     P.run("ffmpm_p2g", prm, ps.n, x.device, ctypes.byref(prm), ctypes.byref(ps), ctypes.byref(g))
-    st.write_back([8, 9])
+    if st is not None:
+        st.write_back([8, 9])
 
 
 def grid_op(grid_resolution, dx, dt, gravity, grid_velocity, grid_mass):
     """three_d/grid_op.py:5-47: momentum -> velocity, gravity, clamp to 0.9 dx/dt, slip walls."""
     dtype = P.dtype_of(grid_velocity)
-    st = E.stage([grid_velocity, grid_mass], dtype=dtype)
-    gv, gm = st.dev
-    E.check_tensors(dtype, gv, gm)
+    (gv, gm), st = P.staged([grid_velocity, grid_mass], dtype)
     prm = E.make_params(3, grid_resolution, dtype, dx, 1.0 / dx, dt, gravity)
     g = E.grid_struct(gv, gm)
     N.call("ffmpm_grid_op", ctypes.byref(prm), ctypes.byref(g), P.stream(gv.device))
-    st.write_back([0])
+    if st is not None:
+        st.write_back([0])
 
 
 def g2p(inv_dx, dt, grid_velocity, particles, v, F, C, Jp, model: str = "neo_hookean"):
     """three_d/g2p.py:9-59: gather v and APIC C, advect, F <- (I + dt C) F."""
     pset, plist = P.split_particles(particles)
     dtype = P.dtype_of(v, F, grid_velocity)
-    st = E.stage([pset.pos, v, F, C, Jp, grid_velocity], dtype=dtype)
-    x, vv, FF, CC, JJ, gv = st.dev
-    E.check_tensors(dtype, x, vv, FF, CC, JJ, gv)
+    (x, vv, FF, CC, JJ, gv), st = P.staged([pset.pos, v, F, C, Jp, grid_velocity], dtype)
     res = gv.shape[0] - 1
     prm = E.make_params(3, res, dtype, 1.0 / inv_dx, inv_dx, dt, model=model)
     ps = E.particles_struct(x, vv, FF, CC, JJ)
     g = E.grid_struct(gv, None)
     P.run("ffmpm_g2p", prm, ps.n, x.device, ctypes.byref(prm), ctypes.byref(g), ctypes.byref(ps))
-    st.write_back([0, 1, 2, 3, 4])
+    if st is not None:
+        st.write_back([0, 1, 2, 3, 4])
     if plist is not None:
         pset.write_positions(plist)
 
@@ -80,12 +78,11 @@ def check_collision_points(points, normals, grid_resolution, dx, grid_velocity, 
     if points.shape != normals.shape:
         raise ValueError("points and normals differ in length")
     dtype = P.dtype_of(grid_velocity)
-    st = E.stage([grid_velocity], dtype=dtype)
-    (gv,) = st.dev
-    E.check_tensors(dtype, gv)
+    (gv,), st = P.staged([grid_velocity], dtype)
     prm = E.make_params(3, grid_resolution, dtype, dx, 1.0 / dx, 1.0, plane_rule=rule)
     pts = np.ascontiguousarray(points)
     nrm = np.ascontiguousarray(normals)
     N.call("ffmpm_check_collision_points", ctypes.byref(prm), pts.ctypes.data_as(ctypes.c_void_p),
            nrm.ctypes.data_as(ctypes.c_void_p), int(len(pts)), ctypes.c_void_p(gv.data_ptr()), P.stream(gv.device))
-    st.write_back([0])
+    if st is not None:
+        st.write_back([0])
