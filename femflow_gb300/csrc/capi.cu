@@ -327,7 +327,7 @@ void sort_and_plan(const ffmpm_params& p, const Layout& L, const Ws& w, const PV
   const uint32_t n = (uint32_t)L.n;
   if (!keys_ready) {
     if (tm) tm->begin(0);
-    k_keys<DIM, T><<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(kp, g, x, n, L.cell_bits, w.keys_next,
+    launch(false, k_keys<DIM, T>, (n + kThreads - 1) / kThreads, kThreads, 0, s, kp, g, x, n, L.cell_bits, w.keys_next,
                                                                        w.block_count, &w.hdr->status);
     if (tm) tm->end(1);
   }
@@ -338,10 +338,10 @@ void sort_and_plan(const ffmpm_params& p, const Layout& L, const Ws& w, const PV
   if (tm) tm->end(1 + L.passes);
   if (tm) tm->begin(2);
   const int ncta = (int)((L.nblocks + kPlanCta - 1) / kPlanCta);
-  k_plan_local<DIM><<<ncta, kPlanCta, 0, s>>>(g, w.block_count, w.block_start, w.block_cnt, w.tmark, w.plan_pref,
+  launch(true, k_plan_local<DIM>, ncta, kPlanCta, 0, s, g, w.block_count, w.block_start, w.block_cnt, w.tmark, w.plan_pref,
                                               w.cta_tot, flag, sym >= 0 ? sym : (flag ? 1 : 0));
-  k_plan_offsets<<<1, kPlanCta, 0, s>>>(w.cta_tot, w.cta_off, ncta, w.hdr, flag);
-  k_plan_write<DIM><<<ncta, kPlanCta, 0, s>>>(g, w.block_count, w.block_start, w.block_cnt, w.tmark, w.plan_pref,
+  launch(true, k_plan_offsets, 1, kPlanCta, 0, s, w.cta_tot, w.cta_off, ncta, w.hdr, flag);
+  launch(true, k_plan_write<DIM>, ncta, kPlanCta, 0, s, g, w.block_count, w.block_start, w.block_cnt, w.tmark, w.plan_pref,
                                               w.cta_off, w.chunks, w.touched, w.occupied, flag);
   if (tm) tm->end(3);
 }
@@ -414,15 +414,15 @@ void launch_p2g_det(const ffmpm_params& p, const Layout& L, const Ws& w, const P
 template <int DIM, typename T>
 void launch_grid_update_det(const ffmpm_params& p, const Layout& L, const Ws& w, cudaStream_t s, T* user_gv = nullptr,
                             T* user_gm = nullptr) {
-  k_grid_update_det<DIM, T><<<work_grid(L.nblocks, 8), kThreads, 0, s>>>(
+  launch(true, k_grid_update_det<DIM, T>, work_grid(L.nblocks, 8), kThreads, 0, s, 
       kparams<T>(p), geom<DIM>(L), w.touched, w.block_cnt, w.hdr, static_cast<const Node4<T>*>(w.stage),
       static_cast<Node4<T>*>(w.gridB), user_gv, user_gm);
 }
 
 template <int DIM, typename T>
-void launch_grid_update(const ffmpm_params& p, const Layout& L, const Ws& w, cudaStream_t s) {
-  k_grid_update<DIM, T><<<work_grid(L.nblocks, 8), kThreads, 0, s>>>(
-      kparams<T>(p), geom<DIM>(L), w.touched, w.hdr, static_cast<Node4<T>*>(w.gridA), static_cast<Node4<T>*>(w.gridB));
+void launch_grid_update(const ffmpm_params& p, const Layout& L, const Ws& w, cudaStream_t s, bool dep = true) {
+  launch(dep, k_grid_update<DIM, T>, work_grid(L.nblocks, 8), kThreads, 0, s, kparams<T>(p), geom<DIM>(L), w.touched, w.hdr,
+         static_cast<Node4<T>*>(w.gridA), static_cast<Node4<T>*>(w.gridB));
 }
 
 template <int DIM, typename T, bool kTma, bool kSorted>
@@ -462,10 +462,10 @@ struct WarpShape {
 
 template <int DIM, typename T>
 void launch_p2g_warp(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, const uint32_t* perm,
-                     int64_t p0, int64_t p1, cudaStream_t s) {
+                     int64_t p0, int64_t p1, cudaStream_t s, bool dep) {
   const WarpShape<T> sh(p1 - p0, 8);
   const size_t smem = sizeof(WarpRecs<DIM, T>) * (sh.threads / 32);
-  k_p2g_warp<DIM, T><<<sh.grid, sh.threads, smem, s>>>(kparams<T>(p), geom<DIM>(L), P, perm, (uint32_t)p0,
+  launch(dep, k_p2g_warp<DIM, T>, sh.grid, sh.threads, smem, s, kparams<T>(p), geom<DIM>(L), P, perm, (uint32_t)p0,
                                                        (uint32_t)p1, static_cast<Node4<T>*>(w.gridA), &w.hdr->status,
                                                        &w.hdr->polar_fallbacks);
 }
@@ -476,7 +476,9 @@ void launch_g2p_sorted(const ffmpm_params& p, const Layout& L, const Ws& w, cons
                        const uint32_t* perm, const G2PExtra& ex, cudaStream_t s) {
   const WarpShape<T> sh(L.n, 8);
   const size_t smem = kNext ? sizeof(WarpRecs<DIM, T>) * (sh.threads / 32) : 0;
-  k_g2p_sorted<DIM, T, kNext><<<sh.grid, sh.threads, smem, s>>>(kparams<T>(p), geom<DIM>(L), Pin, Pout, perm,
+  // plainly: set up early it takes registers from the grid update before it (16,384 particles: 613 us a
+  // 40-substep call, 585 like this; 1M: 4,939 and 4,963)
+  launch(false, k_g2p_sorted<DIM, T, kNext>, sh.grid, sh.threads, smem, s, kparams<T>(p), geom<DIM>(L), Pin, Pout, perm,
                                                                  (uint32_t)L.n, ex, static_cast<Node4<T>*>(w.gridA),
                                                                  w.hdr, w.tmark, w.touched);
 }
@@ -494,31 +496,31 @@ void scatter_unsorted(const ffmpm_params& p, const Layout& L, const Ws& w, const
       uint32_t* rank = w.keys0;
       int* nodes = reinterpret_cast<int*>(w.vals0);
       T* recs = static_cast<T*>(w.recs);
-      k_cell_rank<DIM, T><<<pg, kThreads, 0, s>>>(kp, L.R, P, n, w.cell_count, rank);
-      k_cell_offsets<<<(unsigned)((L.nnodes + kCellTile - 1) / kCellTile), kThreads, 0, s>>>(
+      launch(false, k_cell_rank<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, w.cell_count, rank);
+      launch(true, k_cell_offsets, (unsigned)((L.nnodes + kCellTile - 1) / kCellTile), kThreads, 0, s, 
           w.cell_count, w.cell_start, w.hdr);
-      k_cell_records<DIM, T><<<pg, kThreads, 0, s>>>(kp, L.R, P, n, rank, w.cell_start, recs, nodes, &w.hdr->status,
+      launch(true, k_cell_records<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, rank, w.cell_start, recs, nodes, &w.hdr->status,
                                                      &w.hdr->polar_fallbacks);
       const size_t smem = 2 * sizeof(WarpStage<DIM, T>);
-      k_cell_sums<DIM, T><<<(unsigned)((L.n + 191) / 192), 64, smem, s>>>(L.R, recs, nodes, w.hdr,
+      launch(true, k_cell_sums<DIM, T>, (unsigned)((L.n + 191) / 192), 64, smem, s, L.R, recs, nodes, w.hdr,
                                                                           static_cast<Node4<T>*>(w.gridA));
       return;
     }
   }
-  launch_p2g_warp<DIM, T>(p, L, w, P, nullptr, 0, L.n, s);
+  launch_p2g_warp<DIM, T>(p, L, w, P, nullptr, 0, L.n, s, false);
 }
 
 template <int DIM, typename T>
-void launch_grid_update_dense(const ffmpm_params& p, const Layout& L, const Ws& w, cudaStream_t s) {
-  k_grid_update_dense<DIM, T><<<work_grid((L.nnodes + 4 * kThreads - 1) / (4 * kThreads), 8), kThreads, 0, s>>>(
+void launch_grid_update_dense(const ffmpm_params& p, const Layout& L, const Ws& w, cudaStream_t s, bool dep = true) {
+  launch(dep, k_grid_update_dense<DIM, T>, work_grid((L.nnodes + 4 * kThreads - 1) / (4 * kThreads), 8), kThreads, 0, s, 
       kparams<T>(p), geom<DIM>(L), w.hdr, static_cast<Node4<T>*>(w.gridA), static_cast<Node4<T>*>(w.gridB));
 }
 
 template <int DIM, typename T>
 void launch_g2p_range(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, int64_t p0, int64_t p1,
-                      cudaStream_t s) {
+                      cudaStream_t s, bool dep = true) {
   const WarpShape<T> sh(p1 - p0, 8);
-  k_g2p_range<DIM, T><<<sh.grid, sh.threads, 0, s>>>(kparams<T>(p), geom<DIM>(L), P, (uint32_t)p0, (uint32_t)p1,
+  launch(dep, k_g2p_range<DIM, T>, sh.grid, sh.threads, 0, s, kparams<T>(p), geom<DIM>(L), P, (uint32_t)p0, (uint32_t)p1,
                                                      static_cast<const Node4<T>*>(w.gridB), &w.hdr->status);
 }
 
@@ -655,12 +657,12 @@ int op_substep_host(const ffmpm_params& p, const Layout& L, const Ws& w, const f
     copy(false, a, b, hp->up);
     cudaEventRecord(hp->landed[k], hp->up);
     cudaStreamWaitEvent(s, hp->landed[k], 0);
-    launch_p2g_warp<DIM, T>(p, L, w, pv, nullptr, a, b, s);
+    launch_p2g_warp<DIM, T>(p, L, w, pv, nullptr, a, b, s, false);
   }
-  launch_grid_update_dense<DIM, T>(p, L, w, s);
+  launch_grid_update_dense<DIM, T>(p, L, w, s, false);
   for (int k = 0; k < K; ++k) {
     const int64_t a = lo(k), b = lo(k + 1);
-    launch_g2p_range<DIM, T>(p, L, w, pv, a, b, s);
+    launch_g2p_range<DIM, T>(p, L, w, pv, a, b, s, false);
     cudaEventRecord(hp->gathered[k], s);
     cudaStreamWaitEvent(hp->down, hp->gathered[k], 0);
     copy(true, a, b, hp->down);
@@ -709,7 +711,7 @@ int op_substeps_fused(const ffmpm_params& p, const Layout& L, const Ws& w, PView
   sort_and_plan<DIM, T>(p, L, w, va, false, &sorted_perm, s, tm, nullptr, 1);
   const uint32_t* perm = sorted_perm;  // the permutation the next P2G / G2P applies (null: none)
   if (tm) tm->begin(3);
-  launch_p2g_warp<DIM, T>(p, L, w, va, perm, 0, L.n, s);
+  launch_p2g_warp<DIM, T>(p, L, w, va, perm, 0, L.n, s, true);
   if (tm) tm->end(1);
   for (int k = 0; k < nsteps; ++k) {
     const PView<T>& in = (k & 1) ? vb : va;
@@ -717,7 +719,7 @@ int op_substeps_fused(const ffmpm_params& p, const Layout& L, const Ws& w, PView
     const int32_t* ids_in = (k & 1) ? ids_b : ids_a;
     int32_t* ids_out = (k & 1) ? ids_a : ids_b;
     if (tm) tm->begin(4);
-    launch_grid_update<DIM, T>(p, L, w, s);
+    launch_grid_update<DIM, T>(p, L, w, s, !snap);  // a snapshot's copies lie between
     if (tm) tm->end(1);
     if (k == nsteps - 1) {
       // k >= 1: the buffer is already in the order of the current plan
@@ -789,7 +791,7 @@ int op_p2g(const ffmpm_params& p, const Layout& L, const Ws& w, const ffmpm_part
   const PView<T> pv = pview<T>(*P);
   if (unsorted(p, L)) {
     scatter_unsorted<DIM, T>(p, L, w, pv, s);
-    k_grid_fold_user<DIM, T><<<work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
+    launch(true, k_grid_fold_user<DIM, T>, work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s, 
         L.nnodes, w.hdr, static_cast<Node4<T>*>(w.gridA), static_cast<T*>(grid->velocity),
         static_cast<T*>(grid->mass));
     return check_launch();
@@ -811,7 +813,7 @@ int op_g2p(const ffmpm_params& p, const Layout& L, const Ws& w, const ffmpm_grid
            cudaStream_t s) {
   const PView<T> pv = pview<T>(*P);
   if (unsorted(p, L)) {
-    k_grid_pack_user<DIM, T><<<work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s>>>(
+    launch(false, k_grid_pack_user<DIM, T>, work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s, 
         L.nnodes, static_cast<const T*>(grid->velocity), w.hdr, static_cast<Node4<T>*>(w.gridB));
     launch_g2p_range<DIM, T>(p, L, w, pv, 0, L.n, s);
     return check_launch();
@@ -841,7 +843,7 @@ int op_sort(const ffmpm_params& p, const Layout& L, const Ws& w, const void* x, 
   const uint32_t n = (uint32_t)L.n;
   PView<T> xv{};
   xv.x = static_cast<T*>(const_cast<void*>(x));
-  k_keys<DIM, T><<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(kp, g, xv, n, L.cell_bits, w.keys_next, nullptr,
+  launch(false, k_keys<DIM, T>, (n + kThreads - 1) / kThreads, kThreads, 0, s, kp, g, xv, n, L.cell_bits, w.keys_next, nullptr,
                                                                      &w.hdr->status);
   const uint32_t *ks = nullptr, *perm = nullptr;
   radix_sort(w.keys_next, n, L.passes, w.keys0, w.keys1, w.vals0, w.vals1, w.hist, (int)L.ntiles, &w.hdr->status, s, &ks,

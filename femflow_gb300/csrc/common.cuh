@@ -17,6 +17,35 @@ namespace ffmpm {
 constexpr int kThreads = 256;
 
 // ----------------------------------------------------------------------------------------------
+// Programmatic dependent launch.  The kernels of a substep are short and follow one another; a kernel
+// launched with `dep` may be set up while its predecessor in the stream still runs, and begins with
+// dep_wait, which returns once the predecessor has completed and its writes are visible.  Nothing is read
+// or written before that, and every kernel launched so calls it, so each kernel still sees everything
+// that was launched before it.  The first kernel of an operation, and one that follows a copy, a memset or an
+// event, is launched plainly (dep false), so that what other streams and the copy engines did is waited for
+// in the ordinary way.  8 substeps of 2,048 particles (three kernels each) take 343 us with it and 406
+// without.
+__device__ __forceinline__ void dep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline void launch(bool dep, void (*kern)(P...), int64_t grid, int threads, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dep ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+// ----------------------------------------------------------------------------------------------
 // Precision traits
 template <typename T>
 struct alignas(4 * sizeof(T)) Node4 {

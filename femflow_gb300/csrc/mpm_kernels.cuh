@@ -196,6 +196,7 @@ template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_keys(KParams<T> kp, Geom<DIM> g, PView<T> P, uint32_t n,
                                                    int cell_bits, uint32_t* __restrict__ keys,
                                                    uint32_t* __restrict__ block_count, int32_t* status) {
+  dep_wait();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   bool valid = false;
   uint32_t key = kInvalidKey, blk = 0;
@@ -341,6 +342,7 @@ __global__ void __launch_bounds__(kPlanCta) k_plan_local(Geom<DIM> g, const uint
                                                          uint32_t* __restrict__ block_cnt, uint32_t* __restrict__ tmark,
                                                          uint32_t* __restrict__ pref, Scan4* __restrict__ cta_tot,
                                                          const uint32_t* __restrict__ sort_flag, int sym) {
+  dep_wait();
   if (sort_flag && *sort_flag == 0u) return;
   __shared__ Scan4 part_buf[1][32];
   const int b = blockIdx.x * kPlanCta + threadIdx.x;
@@ -366,6 +368,7 @@ __global__ void __launch_bounds__(kPlanCta) k_plan_local(Geom<DIM> g, const uint
 // One CTA: exclusive prefixes of the CTA totals, and the plan's totals into the header.
 static __global__ void __launch_bounds__(kPlanCta) k_plan_offsets(const Scan4* __restrict__ cta_tot, Scan4* __restrict__ cta_off,
                                                            int ncta, WsHeader* hdr, const uint32_t* __restrict__ sort_flag) {
+  dep_wait();
   if (sort_flag && *sort_flag == 0u) return;
   __shared__ Scan4 part_buf[1][32];
   Scan4 carry{0, 0, 0, 0};
@@ -396,6 +399,7 @@ __global__ void __launch_bounds__(kPlanCta) k_plan_write(Geom<DIM> g, uint32_t* 
                                                          const Scan4* __restrict__ cta_off, int4* __restrict__ chunks,
                                                          uint32_t* __restrict__ touched, int4* __restrict__ occupied,
                                                          const uint32_t* __restrict__ sort_flag) {
+  dep_wait();
   const int b = blockIdx.x * kPlanCta + threadIdx.x;
   if (b >= g.nblocks) return;
   if (!(sort_flag && *sort_flag == 0u)) {
@@ -1165,6 +1169,7 @@ __global__ void __launch_bounds__(kThreads) k_p2g_det(KParams<T> kp, Geom<DIM> g
                                                       const int4* __restrict__ occupied,
                                                       const WsHeader* __restrict__ hdr, Node4<T>* __restrict__ stage,
                                                       int32_t* status, uint32_t* fallbacks, uint32_t* next) {
+  dep_wait();
   if (wait_gave_up(status)) return;
   constexpr int RF = RecLayout<DIM>::kFloats;
   constexpr int RS = RecLayout<DIM>::kStride;
@@ -1488,6 +1493,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_update(KParams<T> kp, Geom<DI
                                                           const uint32_t* __restrict__ touched,
                                                           const WsHeader* __restrict__ hdr, Node4<T>* __restrict__ A,
                                                           Node4<T>* __restrict__ B) {
+  dep_wait();
   const uint32_t nt = hdr->n_touched;
   const int per_block = DIM == 3 ? g.bs * g.bs * g.bs : g.bs * g.bs;
   for (uint32_t tb = blockIdx.x; tb < nt; tb += gridDim.x) {
@@ -1527,6 +1533,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_det(KParams<T> kp, Geo
                                                               const WsHeader* __restrict__ hdr,
                                                               const Node4<T>* __restrict__ stage,
                                                               Node4<T>* __restrict__ B, T* user_gv, T* user_gm) {
+  dep_wait();
   const uint32_t nt = hdr->n_touched;
   const int per_block = DIM == 3 ? g.bs * g.bs * g.bs : g.bs * g.bs;
   const int TN = tile_nodes<DIM>(g);
@@ -1896,6 +1903,7 @@ __global__ void __launch_bounds__(kThreads) k_g2p(KParams<T> kp, Geom<DIM> g, PV
                                                   const WsHeader* __restrict__ hdr, const __grid_constant__ CUtensorMap tmap,
                                                   const T* __restrict__ user_gv, G2PExtra ex, int32_t* status,
                                                   const uint32_t* __restrict__ sort_flag) {
+  dep_wait();
   if (sort_flag && *sort_flag == 0u) perm = nullptr;  // plan kept from an earlier substep: identity order
   if (perm && wait_gave_up(status)) return;
   // Dynamic shared memory: [pad to 128 B][tile: TN Node4][mbarrier].  The TMA destination must

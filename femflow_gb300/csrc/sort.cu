@@ -42,6 +42,7 @@ constexpr int kLookbackBatch = 8;  // predecessor words read per look-back step
 __global__ void __launch_bounds__(kRsThreads) k_radix_ghist(const uint32_t* __restrict__ keys, uint32_t n,
                                                              int passes, uint32_t* __restrict__ ghist,
                                                              const uint32_t* __restrict__ sort_flag) {
+  dep_wait();
   if (sort_flag && *sort_flag == 0u) return;
   __shared__ uint32_t h[kMaxRadixPasses][256];
   for (int i = threadIdx.x; i < kMaxRadixPasses * 256; i += kRsThreads) (&h[0][0])[i] = 0;
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_onesweep(const uint32_t* _
                                                                 uint32_t* __restrict__ vals_out, int32_t* status,
                                                                 const uint32_t* __restrict__ sort_flag,
                                                                 uint32_t wait_limit, uint32_t inject) {
+  dep_wait();
   if (sort_flag && *sort_flag == 0u) return;
   // an earlier pass gave up: this pass's input is incomplete
   if (status && (*reinterpret_cast<const volatile int32_t*>(status) & FFMPM_STATUS_TIMEOUT)) return;
@@ -238,13 +240,13 @@ void radix_sort(const uint32_t* keys_in, uint32_t n, int passes, uint32_t* keys0
   uint32_t* lookback = counters + 32 * passes;  // [passes][ntiles][256]
   cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * radix_scratch_words(passes, ntiles), s);
   const int ghist_grid = std::max(1, std::min(ntiles, 2 * sm_count()));
-  k_radix_ghist<<<ghist_grid, kRsThreads, 0, s>>>(keys_in, n, passes, ghist, sort_flag);
+  launch(false, k_radix_ghist, ghist_grid, kRsThreads, 0, s, keys_in, n, passes, ghist, sort_flag);
   const uint32_t* kin = keys_in;
   const uint32_t* vin = nullptr;
   uint32_t* kbuf[2] = {keys0, keys1};
   uint32_t* vbuf[2] = {vals0, vals1};
   for (int pass = 0; pass < passes; ++pass) {
-    k_radix_onesweep<<<ntiles, kRsThreads, 0, s>>>(kin, vin, n, 8 * pass, ghist + 256 * pass,
+    launch(true, k_radix_onesweep, ntiles, kRsThreads, 0, s, kin, vin, n, 8 * pass, ghist + 256 * pass,
                                                    lookback + (size_t)pass * ntiles * 256, counters + 32 * pass,
                                                    kbuf[pass & 1], vbuf[pass & 1], status, sort_flag, wait_limit,
                                                    inject);

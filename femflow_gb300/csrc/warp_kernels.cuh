@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom
                                                             const uint32_t* __restrict__ perm, uint32_t p0,
                                                             uint32_t p1, Node4<T>* __restrict__ A, int32_t* status,
                                                             uint32_t* fallbacks) {
+  dep_wait();
   if (perm && wait_gave_up(status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpRecs<DIM, T>& wr = reinterpret_cast<WarpRecs<DIM, T>*>(smem_raw)[threadIdx.x >> 5];
@@ -366,6 +367,7 @@ __device__ __forceinline__ int base_node(const KParams<T>& kp, const PView<T>& P
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_cell_rank(KParams<T> kp, int R, PView<T> P, uint32_t n,
                                                         uint32_t* __restrict__ count, uint32_t* __restrict__ rank) {
+  dep_wait();
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   const int node = p < n ? base_node<DIM, T>(kp, P, p, R) : -1;
   const unsigned peers = __match_any_sync(0xffffffffu, node);
@@ -379,6 +381,7 @@ __global__ void __launch_bounds__(kThreads) k_cell_rank(KParams<T> kp, int R, PV
 // count -> start (occupied nodes only); the counters go back to zero for the next call.
 static __global__ void __launch_bounds__(kThreads) k_cell_offsets(uint32_t* __restrict__ count,
                                                                   uint32_t* __restrict__ start, WsHeader* hdr) {
+  dep_wait();
   constexpr int kPer = kCellTile / kThreads;
   static_assert(kPer == 16, "four vectors per thread");
   __shared__ uint32_t warp_sum[kThreads / 32];
@@ -436,6 +439,7 @@ __global__ void __launch_bounds__(kThreads) k_cell_records(KParams<T> kp, int R,
                                                            const uint32_t* __restrict__ start, T* __restrict__ recs,
                                                            int* __restrict__ nodes, int32_t* status,
                                                            uint32_t* fallbacks) {
+  dep_wait();
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   P2GIn<DIM, T> in;
@@ -477,6 +481,7 @@ __device__ __forceinline__ int run_shift(const int* __restrict__ nodes, int at, 
 template <int DIM, typename T>
 __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ recs, const int* __restrict__ nodes,
                                                   const WsHeader* hdr, Node4<T>* __restrict__ A) {
+  dep_wait();
   static_assert(sizeof(T) == 4, "16-byte copies of Node4<float>");
   constexpr int NV = RunRec<DIM>::kPacked / 4, kS = RunRec<DIM>::kSmem, kPitch = WarpStage<DIM, T>::kPitch;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -543,6 +548,7 @@ __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ r
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, Geom<DIM> g, WsHeader* hdr,
                                                                 Node4<T>* __restrict__ A, Node4<T>* __restrict__ B) {
+  dep_wait();
   const int R = g.R;
   const int64_t nn = DIM == 3 ? (int64_t)R * R * R : (int64_t)R * R;
   if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = 0u;  // for the next call's k_cell_offsets
@@ -587,6 +593,7 @@ template <int DIM, typename T>
 __global__ void __launch_bounds__(kWarpCta<T>) k_g2p_range(KParams<T> kp, Geom<DIM> g, PView<T> P, uint32_t p0,
                                                            uint32_t p1, const Node4<T>* __restrict__ B,
                                                            int32_t* status) {
+  dep_wait();
   G2PExtra ex{};
   ex.grid_global = B;
   int org[DIM];
@@ -647,6 +654,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 2 : 1) k_g2p_sor
     KParams<T> kp, Geom<DIM> g, PView<T> Pin, PView<T> Pout, const uint32_t* __restrict__ perm, uint32_t n,
     G2PExtra ex, Node4<T>* __restrict__ A, WsHeader* hdr, uint32_t* __restrict__ tmark,
     uint32_t* __restrict__ touched) {
+  dep_wait();
   int32_t* const status = &hdr->status;
   if (perm && wait_gave_up(status)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -682,6 +690,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 2 : 1) k_g2p_sor
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_fold_user(int64_t nn, WsHeader* hdr, Node4<T>* __restrict__ A, T* __restrict__ gv,
                                                              T* __restrict__ gm) {
+  dep_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = 0u;  // for the next call's k_cell_offsets
   for (int64_t node = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; node < nn;
        node += (int64_t)gridDim.x * blockDim.x) {
@@ -699,6 +708,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_fold_user(int64_t nn, WsHeade
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_pack_user(int64_t nn, const T* __restrict__ gv, WsHeader* hdr,
                                                              Node4<T>* __restrict__ B) {
+  dep_wait();
   for (int64_t node = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; node < nn;
        node += (int64_t)gridDim.x * blockDim.x) {
     T v[3] = {gv[node * DIM + 0], gv[node * DIM + 1], T(0)};
