@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads, sizeof(T) == 4 ? 2 : 1) k_ba
   __shared__ int64_t s_boff[kMaxScenes + 1];
   __shared__ int s_blo0[kMaxScenes], s_blo1[kMaxScenes], s_bw[kMaxScenes];
   __shared__ int s_fail;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   WarpRecs<2, T>& wr = reinterpret_cast<WarpRecs<2, T>*>(smem_raw)[threadIdx.x >> 5];
   const RunLane<2, T> ln;
   if (nsteps <= 0) return;

@@ -104,7 +104,7 @@ bool make_layout(const ffmpm_params& p, int64_t n, Layout* L) {
   L->passes = std::max(1, (L->key_bits + 7) / 8);
   if (L->passes > kMaxRadixPasses) return false;
   L->n = n;
-  L->ntiles = std::max<int64_t>(1, (n + kRadixTile - 1) / kRadixTile);
+  L->ntiles = std::max<int64_t>(1, (n + radix_tile(n) - 1) / radix_tile(n));
   L->max_chunks = (n + kChunk - 1) / kChunk + L->nblocks;
   const size_t node_bytes = size_t(4) * p.real_bytes;
   const int64_t tile_nodes = p.dim == 3 ? int64_t(L->tile) * L->tile * L->tile : int64_t(L->tile) * L->tile;
@@ -333,7 +333,7 @@ void sort_and_plan(const ffmpm_params& p, const Layout& L, const Ws& w, const PV
   }
   const uint32_t* ks = nullptr;
   if (tm) tm->begin(1);
-  radix_sort(w.keys_next, n, L.passes, w.keys0, w.keys1, w.vals0, w.vals1, w.hist, (int)L.ntiles, &w.hdr->status, s,
+  radix_sort(w.keys_next, n, L.passes, w.keys0, w.keys1, w.vals0, w.vals1, w.hist, radix_tile(L.n), &w.hdr->status, s,
              &ks, perm, flag, p.wait_limit, p.inject);
   if (tm) tm->end(1 + L.passes);
   if (tm) tm->begin(2);
@@ -771,12 +771,18 @@ int op_substeps_sorted(const ffmpm_params& p, const Layout& L, const Ws& w, ffmp
     else
       launch_grid_update<DIM, T>(p, L, w, s);
     if (tm) tm->end(1);
-    G2PExtra ex{ids_in, ids_out, w.keys_next, w.block_count, L.cell_bits, flag ? w.gridB : nullptr,
-                flag ? &w.hdr->far_stray : nullptr};
+    G2PExtra ex{ids_in, ids_out, w.keys_next, w.block_count, L.cell_bits, w.gridB, flag ? &w.hdr->far_stray : nullptr};
     if (tm) tm->begin(5);
-    int rc = launch_g2p<DIM, T, true, true>(p, L, w, in, out, perm, nullptr, ex, s, flag);
+    if (p.deterministic) {
+      // by warps, not by chunks of the 4^3 blocks, a fifth of whose slots are empty (particle by particle the
+      // same sums, bit for bit)
+      launch_g2p_sorted<DIM, T, false>(p, L, w, in, out, perm, ex, s);
+    } else {
+      if (!flag) ex.grid_global = nullptr;
+      const int rc = launch_g2p<DIM, T, true, true>(p, L, w, in, out, perm, nullptr, ex, s, flag);
+      if (rc != FFMPM_OK) return rc;
+    }
     if (tm) tm->end(1);
-    if (rc != FFMPM_OK) return rc;
     snapshot<DIM, T>(snap, k, out, ids_out, L.n, s);
   }
   // The last G2P counted the blocks of the final state for a substep that will not run here:
@@ -846,7 +852,7 @@ int op_sort(const ffmpm_params& p, const Layout& L, const Ws& w, const void* x, 
   launch(false, k_keys<DIM, T>, (n + kThreads - 1) / kThreads, kThreads, 0, s, kp, g, xv, n, L.cell_bits, w.keys_next, nullptr,
                                                                      &w.hdr->status);
   const uint32_t *ks = nullptr, *perm = nullptr;
-  radix_sort(w.keys_next, n, L.passes, w.keys0, w.keys1, w.vals0, w.vals1, w.hist, (int)L.ntiles, &w.hdr->status, s, &ks,
+  radix_sort(w.keys_next, n, L.passes, w.keys0, w.keys1, w.vals0, w.vals1, w.hist, radix_tile(L.n), &w.hdr->status, s, &ks,
              &perm, nullptr, p.wait_limit, p.inject);
   if (keys_out) cudaMemcpyAsync(keys_out, ks, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
   if (perm_out) cudaMemcpyAsync(perm_out, perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);

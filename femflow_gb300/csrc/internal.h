@@ -11,7 +11,8 @@ namespace ffmpm {
 
 constexpr uint32_t kInvalidKey = 0xFFFFFFFFu;
 constexpr int kChunk = 512;       // particles per P2G/G2P work item
-constexpr int kRadixTile = 4096;  // keys per radix-sort CTA (256 threads x 16)
+constexpr int kRadixTile = 4096;  // most keys per radix-sort CTA (256 threads x 16)
+int radix_tile(int64_t n);        // keys per CTA for n keys
 
 // Workspace header: status word, counters, polar fallbacks.
 struct WsHeader {
@@ -53,7 +54,7 @@ int sm_count();
 constexpr int kMaxRadixPasses = 4;
 size_t radix_scratch_words(int passes, int64_t ntiles);
 void radix_sort(const uint32_t* keys_in, uint32_t n, int passes, uint32_t* keys0, uint32_t* keys1, uint32_t* vals0,
-                uint32_t* vals1, uint32_t* scratch, int ntiles, int32_t* status, cudaStream_t s,
+                uint32_t* vals1, uint32_t* scratch, int tile, int32_t* status, cudaStream_t s,
                 const uint32_t** keys_sorted, const uint32_t** perm, const uint32_t* sort_flag = nullptr,
                 uint32_t wait_limit = 0, uint32_t inject = 0);
 

@@ -107,7 +107,7 @@ void sort_static(const ffmpm_params& p, const Layout& L, uint32_t* base, const v
   k_keys<DIM, T><<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(kp, g, xv, n, L.cell_bits, keys_next, nullptr,
                                                                      status);
   const uint32_t *ks = nullptr, *perm = nullptr;
-  radix_sort(keys_next, n, L.passes, keys0, keys1, vals0, vals1, hist, (int)L.ntiles, status, s, &ks, &perm, nullptr,
+  radix_sort(keys_next, n, L.passes, keys0, keys1, vals0, vals1, hist, kRadixTile, status, s, &ks, &perm, nullptr,
              p.wait_limit, p.inject);
   if (keys_out) cudaMemcpyAsync(keys_out, ks, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
   if (perm_out) cudaMemcpyAsync(perm_out, perm, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
@@ -124,7 +124,7 @@ extern "C" int ffmpm_sort_by_block_static(const ffmpm_params* p, const void* x, 
   if (n > kStaticMaxN) return FFMPM_ERR_CAPACITY;
   Layout L;
   if (!p || !make_layout(*p, n, &L)) return FFMPM_ERR_BADARG;
-  if (L.ntiles > kStaticTiles) return FFMPM_ERR_CAPACITY;
+  if ((n + kRadixTile - 1) / kRadixTile > kStaticTiles) return FFMPM_ERR_CAPACITY;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (n == 0) {
     if (status_out) return cudaMemsetAsync(status_out, 0, sizeof(int32_t), s) == cudaSuccess ? FFMPM_OK : FFMPM_ERR_CUDA;

@@ -26,9 +26,7 @@ namespace ffmpm {
 namespace {
 
 constexpr int kRsThreads = 256;
-constexpr int kRsItems = 16;
 constexpr int kRsWarps = kRsThreads / 32;
-static_assert(kRsThreads * kRsItems == kRadixTile, "tile size");
 
 // Published look-back word: 2 flag bits over a 30-bit count (n < 2^30).
 constexpr uint32_t kFlagAggregate = 1u << 30;
@@ -39,6 +37,7 @@ constexpr int kLookbackBatch = 8;  // predecessor words read per look-back step
 
 // Digit histograms of all passes (ghist[pass][256]), one read of the keys.  Nearly sorted keys put
 // equal digits in neighbouring lanes, so each warp first merges equal digits (__match_any_sync).
+template <int kRsItems>
 __global__ void __launch_bounds__(kRsThreads) k_radix_ghist(const uint32_t* __restrict__ keys, uint32_t n,
                                                              int passes, uint32_t* __restrict__ ghist,
                                                              const uint32_t* __restrict__ sort_flag) {
@@ -48,9 +47,10 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_ghist(const uint32_t* __re
   for (int i = threadIdx.x; i < kMaxRadixPasses * 256; i += kRsThreads) (&h[0][0])[i] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  // each CTA takes whole 4096-key tiles; a thread's 16 keys are loaded before any is counted
-  for (uint32_t tile = blockIdx.x; tile * (uint32_t)kRadixTile < n; tile += gridDim.x) {
-    const uint32_t base = tile * (uint32_t)kRadixTile + threadIdx.x;
+  constexpr uint32_t kTile = kRsThreads * kRsItems;
+  // each CTA takes whole tiles; a thread's keys are loaded before any is counted
+  for (uint32_t tile = blockIdx.x; tile * kTile < n; tile += gridDim.x) {
+    const uint32_t base = tile * kTile + threadIdx.x;
     uint32_t k[kRsItems];
 #pragma unroll
     for (int r = 0; r < kRsItems; ++r) {
@@ -79,6 +79,7 @@ __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {
 }
 __device__ __forceinline__ void st_volatile(uint32_t* p, uint32_t v) { *reinterpret_cast<volatile uint32_t*>(p) = v; }
 
+template <int kRsItems>
 __global__ void __launch_bounds__(kRsThreads) k_radix_onesweep(const uint32_t* __restrict__ keys_in,
                                                                 const uint32_t* __restrict__ vals_in, uint32_t n,
                                                                 int shift, const uint32_t* __restrict__ ghist,
@@ -121,8 +122,8 @@ __global__ void __launch_bounds__(kRsThreads) k_radix_onesweep(const uint32_t* _
   }
   __syncthreads();
   const uint32_t tile = s_tile;
-  // rank: warp w handles keys [tile*4096 + w*512, +512) in 16 rounds of 32, in index order
-  const uint32_t sub = tile * (uint32_t)kRadixTile + warp * (kRsItems * 32);
+  // rank: warp w handles its kRsItems * 32 neighbouring keys of the tile in rounds of 32, in index order
+  const uint32_t sub = tile * (uint32_t)(kRsThreads * kRsItems) + warp * (kRsItems * 32);
   const unsigned lt = lanemask_lt();
   uint32_t key[kRsItems], val[kRsItems], off[kRsItems], dig[kRsItems];
   // all of this thread's keys and values are loaded before the ranking starts
@@ -230,31 +231,52 @@ size_t radix_scratch_words(int passes, int64_t ntiles) {
   return size_t(passes) * (256 + 32 + 256 * size_t(ntiles));
 }
 
-void radix_sort(const uint32_t* keys_in, uint32_t n, int passes, uint32_t* keys0, uint32_t* keys1, uint32_t* vals0,
-                uint32_t* vals1, uint32_t* scratch, int ntiles, int32_t* status, cudaStream_t s,
-                const uint32_t** keys_sorted, const uint32_t** perm, const uint32_t* sort_flag, uint32_t wait_limit,
-                uint32_t inject) {
-  if (wait_limit == 0) wait_limit = kLookbackSpins;
+// Keys per tile for n keys: a quarter or half of the largest while the tiles then still fit the SMs in one
+// wave.  A tile's ranking is a chain of rounds, so that small sorts are faster in more, smaller tiles; large
+// ones take the fewest tiles to look back over.  40 substeps of 16,384 particles, five sorts: 585 -> 546 us;
+// 20 deterministic substeps of 300,000 particles, a sort each (and their G2P by warps): 2,320 -> 2,124.
+int radix_tile(int64_t n) {
+  const int64_t sms = 148;  // by n alone: a workspace's size must not depend on the device
+  if (n <= sms * kRadixTile / 4) return kRadixTile / 4;
+  if (n <= sms * kRadixTile / 2) return kRadixTile / 2;
+  return kRadixTile;
+}
+
+template <int kItems>
+static void radix_passes(const uint32_t* keys_in, uint32_t n, int passes, uint32_t* const kbuf[2], uint32_t* const vbuf[2],
+                         uint32_t* scratch, int ntiles, int32_t* status, cudaStream_t s, const uint32_t* sort_flag,
+                         uint32_t wait_limit, uint32_t inject) {
   uint32_t* ghist = scratch;                    // [passes][256]
   uint32_t* counters = ghist + 256 * passes;    // [passes], 32-word padded
   uint32_t* lookback = counters + 32 * passes;  // [passes][ntiles][256]
-  cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * radix_scratch_words(passes, ntiles), s);
   const int ghist_grid = std::max(1, std::min(ntiles, 2 * sm_count()));
-  launch(false, k_radix_ghist, ghist_grid, kRsThreads, 0, s, keys_in, n, passes, ghist, sort_flag);
+  launch(false, k_radix_ghist<kItems>, ghist_grid, kRsThreads, 0, s, keys_in, n, passes, ghist, sort_flag);
   const uint32_t* kin = keys_in;
   const uint32_t* vin = nullptr;
-  uint32_t* kbuf[2] = {keys0, keys1};
-  uint32_t* vbuf[2] = {vals0, vals1};
   for (int pass = 0; pass < passes; ++pass) {
-    launch(true, k_radix_onesweep, ntiles, kRsThreads, 0, s, kin, vin, n, 8 * pass, ghist + 256 * pass,
-                                                   lookback + (size_t)pass * ntiles * 256, counters + 32 * pass,
-                                                   kbuf[pass & 1], vbuf[pass & 1], status, sort_flag, wait_limit,
-                                                   inject);
+    launch(true, k_radix_onesweep<kItems>, ntiles, kRsThreads, 0, s, kin, vin, n, 8 * pass, ghist + 256 * pass,
+           lookback + (size_t)pass * ntiles * 256, counters + 32 * pass, kbuf[pass & 1], vbuf[pass & 1], status, sort_flag,
+           wait_limit, inject);
     kin = kbuf[pass & 1];
     vin = vbuf[pass & 1];
   }
-  *keys_sorted = kin;
-  *perm = vin;
+}
+
+void radix_sort(const uint32_t* keys_in, uint32_t n, int passes, uint32_t* keys0, uint32_t* keys1, uint32_t* vals0,
+                uint32_t* vals1, uint32_t* scratch, int tile, int32_t* status, cudaStream_t s,
+                const uint32_t** keys_sorted, const uint32_t** perm, const uint32_t* sort_flag, uint32_t wait_limit,
+                uint32_t inject) {
+  if (wait_limit == 0) wait_limit = kLookbackSpins;
+  const int ntiles = (int)std::max<int64_t>(1, (int64_t(n) + tile - 1) / tile);
+  cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * radix_scratch_words(passes, ntiles), s);
+  uint32_t* const kbuf[2] = {keys0, keys1};
+  uint32_t* const vbuf[2] = {vals0, vals1};
+  const auto run = tile == kRadixTile / 4   ? radix_passes<kRadixTile / 4 / kRsThreads>
+                   : tile == kRadixTile / 2 ? radix_passes<kRadixTile / 2 / kRsThreads>
+                                            : radix_passes<kRadixTile / kRsThreads>;
+  run(keys_in, n, passes, kbuf, vbuf, scratch, ntiles, status, s, sort_flag, wait_limit, inject);
+  *keys_sorted = kbuf[(passes - 1) & 1];
+  *perm = vbuf[(passes - 1) & 1];
 }
 
 }  // namespace ffmpm

@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom
                                                             uint32_t* fallbacks) {
   dep_wait();
   if (perm && wait_gave_up(status)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   WarpRecs<DIM, T>& wr = reinterpret_cast<WarpRecs<DIM, T>*>(smem_raw)[threadIdx.x >> 5];
   const RunLane<DIM, T> ln;
   const int lane = threadIdx.x & 31;
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ r
   dep_wait();
   static_assert(sizeof(T) == 4, "16-byte copies of Node4<float>");
   constexpr int NV = RunRec<DIM>::kPacked / 4, kS = RunRec<DIM>::kSmem, kPitch = WarpStage<DIM, T>::kPitch;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   WarpStage<DIM, T>& ws = reinterpret_cast<WarpStage<DIM, T>*>(smem_raw)[threadIdx.x >> 5];
   const RunLane<DIM, T> ln;
   const int lane = threadIdx.x & 31;
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 2 : 1) k_g2p_sor
   dep_wait();
   int32_t* const status = &hdr->status;
   if (perm && wait_gave_up(status)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   WarpRecs<DIM, T>& wr = reinterpret_cast<WarpRecs<DIM, T>*>(smem_raw)[kNext ? threadIdx.x >> 5 : 0];
   const RunLane<DIM, T> ln;
   const int lane = threadIdx.x & 31;
