@@ -146,11 +146,15 @@ class MPMRollout(torch.autograd.Function):
     about 1e-2 of the total at 1e5 particles)."""
 
     @staticmethod
-    def forward(ctx, x0, v0, F0, C0, mu_0, lambda_0, mass, cfg: RolloutConfig):
+    def forward(ctx, x0, v0, F0, C0, mu_0, lambda_0, mass, cfg: RolloutConfig, perm=None, inv=None):
+        """``perm`` (with its inverse ``inv``): the order the rollout runs on; the packed state is gathered
+        once each way, so that the caller's arrays and gradients stay in their own order."""
         n = x0.shape[0]
         ctx.scalar_mu, ctx.scalar_lam = mu_0.dim() == 0, lambda_0.dim() == 0
-        runner = _Runner(cfg, n, x0.dtype, x0.device, mass, mu_0.expand(n), lambda_0.expand(n), dim=x0.shape[1])
-        buf = pack(x0.detach(), v0.detach(), F0.detach(), C0.detach())
+        pick = lambda t: t if perm is None or not torch.is_tensor(t) or t.dim() == 0 or t.shape[0] != n else t[perm]
+        runner = _Runner(cfg, n, x0.dtype, x0.device, pick(mass), pick(mu_0.detach()).expand(n),
+                         pick(lambda_0.detach()).expand(n), dim=x0.shape[1])
+        buf = _gather(pack(x0.detach(), v0.detach(), F0.detach(), C0.detach()), perm)
         K = max(1, int(cfg.checkpoint_every))
         ckpts = []
         for s in range(cfg.steps):
@@ -158,8 +162,8 @@ class MPMRollout(torch.autograd.Function):
                 ckpts.append(buf.clone())
             runner.substep(buf)
         runner.check()
-        ctx.runner, ctx.ckpts, ctx.cfg = runner, ckpts, cfg
-        return unpack(buf)
+        ctx.runner, ctx.ckpts, ctx.cfg, ctx.perm, ctx.inv = runner, ckpts, cfg, perm, inv
+        return unpack(_gather(buf, inv))
 
     @staticmethod
     def backward(ctx, gx, gv, gF, gC):
@@ -170,7 +174,7 @@ class MPMRollout(torch.autograd.Function):
             return torch.zeros(shape, dtype=dtype, device=dev) if g is None else g.to(dtype)
 
         d = runner.dim
-        adj = pack(z(gx, (n, d)), z(gv, (n, d)), z(gF, (n, d, d)), z(gC, (n, d, d)))
+        adj = _gather(pack(z(gx, (n, d)), z(gv, (n, d)), z(gF, (n, d, d)), z(gC, (n, d, d))), ctx.perm)
         mu_bar = torch.zeros(n, dtype=torch.float64, device=dev)
         lam_bar = torch.zeros(n, dtype=torch.float64, device=dev)
         K = max(1, int(cfg.checkpoint_every))
@@ -184,17 +188,25 @@ class MPMRollout(torch.autograd.Function):
             for k in reversed(range(count)):
                 runner.adjoint(seg[k], adj, mu_bar, lam_bar)
         runner.check()
-        gx0, gv0, gF0, gC0 = unpack(adj)
-        ctx.runner = ctx.ckpts = None
-        g_mu = mu_bar.sum() if ctx.scalar_mu else mu_bar
-        g_lam = lam_bar.sum() if ctx.scalar_lam else lam_bar
-        return gx0, gv0, gF0, gC0, g_mu.to(dtype), g_lam.to(dtype), None, None
+        gx0, gv0, gF0, gC0 = unpack(_gather(adj, ctx.inv))
+        back = lambda t: t if ctx.inv is None else t[ctx.inv]
+        g_mu = mu_bar.sum() if ctx.scalar_mu else back(mu_bar)
+        g_lam = lam_bar.sum() if ctx.scalar_lam else back(lam_bar)
+        ctx.runner = ctx.ckpts = ctx.perm = ctx.inv = None
+        return (gx0, gv0, gF0, gC0, g_mu.to(dtype), g_lam.to(dtype)) + (None,) * (len(ctx.needs_input_grad) - 6)
+
+
+def _gather(buf: torch.Tensor, perm) -> torch.Tensor:
+    """The columns of a component-major buffer in the order ``perm`` (None: as they are)."""
+    return buf if perm is None else buf.index_select(1, perm)
 
 
 def cell_order(x: torch.Tensor, res: int) -> torch.Tensor:
     """Stable order of particles by base cell (the node a particle's stencil starts at)."""
     R = res + 1
-    b = torch.clamp(torch.floor(x.detach() * res - 0.5), -1, res).to(torch.int64) + 1
+    # 32-bit keys where they suffice: half the passes of a 64-bit sort
+    kind = torch.int32 if (R + 2) ** x.shape[1] < 2 ** 31 else torch.int64
+    b = torch.clamp(torch.floor(x.detach() * res - 0.5), -1, res).to(kind) + 1
     key = b[:, 0]
     for a in range(1, x.shape[1]):
         key = key * (R + 2) + b[:, a]
@@ -210,7 +222,7 @@ def simulate(x0, v0, mu_0, lambda_0, cfg: RolloutConfig, mass, F0=None, C0=None,
     F0, C0 default to the reference's initial state (identity, zero; mls_mpm.py:9-15).
     With ``order`` the rollout runs on the particles ordered by base cell (neighbouring lanes of the
     adjoint kernels then share stencil nodes); inputs and outputs stay in the caller's order, and
-    autograd carries the permutation.
+    the rollout's state is gathered once each way.
     """
     n, d = x0.shape[0], x0.shape[1]
     dtype, dev = x0.dtype, x0.device
@@ -225,7 +237,5 @@ def simulate(x0, v0, mu_0, lambda_0, cfg: RolloutConfig, mass, F0=None, C0=None,
     perm = cell_order(x0, cfg.res)
     inv = torch.empty_like(perm)
     inv[perm] = torch.arange(n, device=perm.device)
-    pick = lambda t: t[perm] if torch.is_tensor(t) and t.dim() >= 1 and t.shape[0] == n else t
     cfg = replace(cfg, cell_order=True)
-    out = MPMRollout.apply(pick(x0), pick(v0), pick(F0), pick(C0), pick(mu), pick(lam), pick(mass), cfg)
-    return tuple(o[inv] for o in out)
+    return MPMRollout.apply(x0, v0, F0, C0, mu, lam, mass, cfg, perm, inv)
