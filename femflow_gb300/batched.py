@@ -97,7 +97,8 @@ class Batch2D:
         self.ws = (self._wsbuf.data_ptr() + 255) // 256 * 256
         N.call("ffmpm_batch2d_init", tptr, self.nscenes, self.rb, ctypes.c_void_p(self.ws),
                ctypes.c_size_t(self.ws_bytes), ctypes.c_void_p(E._stream_ptr(self.device)))
-        self.threads, self.ctas_per_sm = 256, 0
+        # float32, 4 scenes to 256: 0 to 6 % faster than 256 threads (fewer CTAs at the barriers)
+        self.threads, self.ctas_per_sm = (512 if self.rb == 4 else 256), 0
         self._graph, self._graph_steps = None, 0
 
     def _struct(self):

@@ -563,7 +563,10 @@ int ffmpm_batch2d_substeps(int32_t nscenes, int32_t real_bytes, ffmpm_particles*
       return FFMPM_ERR_CUDA;
     }
     if (ctas_per_sm > 0) per_sm = std::min(per_sm, (int)ctas_per_sm);
-    const int grid = per_sm * sm_count();  // every CTA resident: the cooperative launch checks it
+    // every CTA resident (the cooperative launch checks it); no more than the particles fill beyond one per SM:
+    // the others would only add to the barriers
+    const int64_t fill = std::max<int64_t>(sm_count(), (P->n + nt - 1) / nt);
+    const int grid = (int)std::min<int64_t>(int64_t(per_sm) * sm_count(), fill);
     unsigned char* wsp = static_cast<unsigned char*>(ws);
     // a launch whose barrier ran out leaves its arrivals counted: start every call from zero
     if (cudaMemsetAsync(wsp + offsetof(BatchHeader, barrier_count), 0, sizeof(uint32_t), s) != cudaSuccess)
