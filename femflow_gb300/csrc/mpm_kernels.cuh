@@ -1602,22 +1602,24 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_det(KParams<T> kp, Geo
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_op_dense(KParams<T> kp, int R, T* __restrict__ gv,
                                                             const T* __restrict__ gm) {
-  const int64_t nn = DIM == 3 ? (int64_t)R * R * R : (int64_t)R * R;
-  for (int64_t node = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; node < nn;
-       node += (int64_t)gridDim.x * blockDim.x) {
+  // below 2^31 nodes (the sort keys bound the grid): 32-bit divisions, the 64-bit ones were most of the
+  // kernel (2.1M nodes: 15.3 -> 11.2 us)
+  const uint32_t nn = DIM == 3 ? (uint32_t)R * R * R : (uint32_t)R * R, Ru = (uint32_t)R;
+  for (uint32_t node = blockIdx.x * blockDim.x + threadIdx.x; node < nn; node += gridDim.x * blockDim.x) {
     int I[DIM];
     if constexpr (DIM == 3) {
-      I[0] = (int)(node / ((int64_t)R * R));
-      I[1] = (int)((node / R) % R);
-      I[2] = (int)(node % R);
+      I[0] = (int)(node / (Ru * Ru));
+      I[1] = (int)((node / Ru) % Ru);
+      I[2] = (int)(node % Ru);
     } else {
-      I[0] = (int)(node / R);
-      I[1] = (int)(node % R);
+      I[0] = (int)(node / Ru);
+      I[1] = (int)(node % Ru);
     }
-    T vel[3] = {gv[node * DIM + 0], gv[node * DIM + 1], DIM == 3 ? gv[node * DIM + DIM - 1] : T(0)};
+    const size_t at = (size_t)node * DIM;
+    T vel[3] = {gv[at + 0], gv[at + 1], DIM == 3 ? gv[at + DIM - 1] : T(0)};
     grid_node<DIM, T>(kp, I, vel, gm[node]);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) gv[node * DIM + d] = vel[d];
+    for (int d = 0; d < DIM; ++d) gv[at + d] = vel[d];
   }
 }
 

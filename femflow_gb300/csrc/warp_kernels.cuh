@@ -348,7 +348,8 @@ __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom
 // 1,048,576 particles of a random order on 128^3, component-major (GB300): 18 + 5 + 79 + 50 us, where
 // the block sort and the chunked scatter through its permutation took 150 + 305 us (every component
 // of a particle then came from a sector of its own).  k_cell_records is bound by its scattered 64-byte
-// record writes, k_cell_sums by instruction issue.
+// record writes and wants the warps that 80 registers allow (a coarse step of 552 us takes 540 with them),
+// k_cell_sums by instruction issue.
 constexpr int kCellTile = 4096;      // nodes per CTA of k_cell_offsets
 constexpr uint32_t kNoRank = 0xffffffffu;
 
@@ -434,7 +435,7 @@ static __global__ void __launch_bounds__(kThreads) k_cell_offsets(uint32_t* __re
 }
 
 template <int DIM, typename T>
-__global__ void __launch_bounds__(kThreads) k_cell_records(KParams<T> kp, int R, PView<T> P, uint32_t n,
+__global__ void __launch_bounds__(kThreads, 3) k_cell_records(KParams<T> kp, int R, PView<T> P, uint32_t n,
                                                            const uint32_t* __restrict__ rank,
                                                            const uint32_t* __restrict__ start, T* __restrict__ recs,
                                                            int* __restrict__ nodes, int32_t* status,
@@ -590,7 +591,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, G
 
 // G2P of particles [p0, p1) in place, every stencil gathered from the global velocity grid B.
 template <int DIM, typename T>
-__global__ void __launch_bounds__(kWarpCta<T>) k_g2p_range(KParams<T> kp, Geom<DIM> g, PView<T> P, uint32_t p0,
+__global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 3 : 1) k_g2p_range(KParams<T> kp, Geom<DIM> g, PView<T> P, uint32_t p0,
                                                            uint32_t p1, const Node4<T>* __restrict__ B,
                                                            int32_t* status) {
   dep_wait();
