@@ -1,6 +1,7 @@
 // MLS-MPM substep kernels, templated on dimension (2, 3) and precision (float, double).
 //
-// Pipeline of one substep (all on one stream):
+// Pipeline of one block-sorted substep (all on one stream; the kernels of warp_kernels.cuh take the
+// place of k_p2g_cells and k_g2p in the resident solver, and need no sort on arrays in place):
 //   k_keys         block key of every particle (three_d/p2g.py:50 base rule) + block histogram
 //   radix sort     stable, bit-exact permutation by key (sort.cu)
 //   k_plan_*       block offsets, work chunks, touched-block list (three launches)

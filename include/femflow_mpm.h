@@ -168,7 +168,7 @@ int ffmpm_substep(const ffmpm_params *p, ffmpm_particles *P, void *ws, size_t ws
  * lambda_0 only where the host gives them), the substep runs there, and x, v, F, C, Jp come back
  * into the host arrays.  Uploads and the scatter, and the gather and the downloads, are pipelined
  * over chunks of particles: each chunk is scattered in the caller's order as soon as it has landed
- * (one vector atomic per node, no block sort), the grid update covers every node, and each chunk
+ * (no sort), the grid update covers every node, and each chunk
  * is gathered and sent back while the next one is gathered.  Same arithmetic per particle as
  * ffmpm_substep; the node sums run in another order.  The deterministic mode uploads everything,
  * runs ffmpm_substep and downloads.  The copies use two streams and a few events of the library's
@@ -391,8 +391,9 @@ int ffmpm_corrector_g2p(const ffmpm_params *p, const ffmpm_grid *grid, ffmpm_par
  *   W1 at 0 (rows of 128, 64 used), W2 at 16384, W3 at 24576, W4 at 32768 (rows of 64; W2, W3: 64
  *   rows used; W4: 12), b1 at 40960, b2 at 41024, b3 at 41088, b4 at 41152 (16).
  * Activation buffers are sized for max_batch rows (a multiple of 128); transposed buffers are
- * strided by the batch of the call and their padding rows (Xt rows 113.., dYt rows 12.., dZt rows
- * 64..) are zeroed by the calls themselves.  All buffers are caller allocated. */
+ * strided by the batch of the call; Xt's padding rows (113..) are zeroed by the forward pass.  All
+ * buffers are caller allocated.  dH, dY, dZ, dYt and dZt are no longer used (the backward pass keeps
+ * them on the chip). */
 #define FFMPM_MLP_PARAMS 41168
 #define FFMPM_MLP_OFF_W1 0
 #define FFMPM_MLP_OFF_W2 16384
