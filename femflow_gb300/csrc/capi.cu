@@ -821,7 +821,7 @@ int op_g2p(const ffmpm_params& p, const Layout& L, const Ws& w, const ffmpm_grid
   const PView<T> pv = pview<T>(*P);
   if (unsorted(p, L)) {
     launch(false, k_grid_pack_user<DIM, T>, work_grid((L.nnodes + kThreads - 1) / kThreads, 8), kThreads, 0, s, 
-        L.nnodes, static_cast<const T*>(grid->velocity), w.hdr, static_cast<Node4<T>*>(w.gridB));
+        L.nnodes, static_cast<const T*>(grid->velocity), static_cast<Node4<T>*>(w.gridB));
     launch_g2p_range<DIM, T>(p, L, w, pv, 0, L.n, s);
     return check_launch();
   }

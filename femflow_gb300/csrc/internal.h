@@ -25,10 +25,9 @@ struct WsHeader {
   uint32_t sort_now;   // sort cadence: 1 when this substep re-sorts (set by k_sort_decide)
   uint32_t far_stray;  // set by G2P when a particle left the neighbourhood its block's plan covers
   uint32_t det_next[2];  // deterministic P2G: next entry of the occupied list, per pass (zeroed per launch)
-  uint32_t b_dirty;  // the velocity grid has held a non-finite value (see k_grid_update_dense)
   uint32_t cell_cursor;  // slots handed out by k_cell_offsets (zeroed by the grid pass that follows)
   uint32_t cell_occupied;  // cells with particles, as counted by k_cell_offsets (zeroed with it)
-  uint32_t pad[51];
+  uint32_t pad[52];
 };
 static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
 

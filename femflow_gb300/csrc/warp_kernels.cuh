@@ -542,10 +542,10 @@ __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ r
 }
 
 // Grid update of every node (three_d/grid_op.py:5-47 / two_d/grid_op.py:5-24): momentum of A ->
-// velocity in B, A re-zeroed.  Nodes that received nothing are skipped: their B is read by no
-// particle, or with weight zero (a particle half a cell from its neighbours).  Weight zero times a
-// value left by an earlier substep is zero as long as that value is finite, so the first update that
-// writes a non-finite velocity raises hdr->b_dirty, and from then on skipped nodes get zeros.
+// velocity in B, A re-zeroed.  B is written at every node: one whose sums are all zero has velocity zero, and
+// particles do read it (without mass and stress at full weight; half a cell from their neighbours at weight
+// zero, which an infinity left there by an earlier call would still spoil).  Writing it (450,000 particles on
+// 128^3, four substeps: 840 us, 834 without) is cheaper than to read first whether it holds a value (854).
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, Geom<DIM> g, WsHeader* hdr,
                                                                 Node4<T>* __restrict__ A, Node4<T>* __restrict__ B) {
@@ -553,7 +553,6 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, G
   const int R = g.R;
   const int64_t nn = DIM == 3 ? (int64_t)R * R * R : (int64_t)R * R;
   if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = 0u;  // for the next call's k_cell_offsets
-  const bool sweep = *reinterpret_cast<const volatile uint32_t*>(&hdr->b_dirty) != 0u;
   constexpr int U = 4;  // nodes of a thread in flight
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t n0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n0 < nn; n0 += U * stride) {
@@ -567,7 +566,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, G
     for (int u = 0; u < U; ++u) {
       const int64_t node = n0 + u * stride;
       if (a[u].x == T(0) && a[u].y == T(0) && a[u].z == T(0) && a[u].w == T(0)) {
-        if (sweep && node < nn) B[node] = Node4<T>{T(0), T(0), T(0), T(0)};
+        if (node < nn) B[node] = Node4<T>{T(0), T(0), T(0), T(0)};
         continue;
       }
       int I[DIM];
@@ -582,7 +581,6 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, G
       }
       T vel[3] = {a[u].x, a[u].y, a[u].z};
       grid_node<DIM, T>(kp, I, vel, a[u].w);
-      if (nonfinite_probe(vel, 3) != T(0)) hdr->b_dirty = 1u;
       B[node] = Node4<T>{vel[0], vel[1], vel[2], a[u].w};
       A[node] = Node4<T>{T(0), T(0), T(0), T(0)};
     }
@@ -707,14 +705,13 @@ __global__ void __launch_bounds__(kThreads) k_grid_fold_user(int64_t nn, WsHeade
 
 // A caller's grid_velocity [nodes][DIM] into the workspace's B (one aligned vector per node).
 template <int DIM, typename T>
-__global__ void __launch_bounds__(kThreads) k_grid_pack_user(int64_t nn, const T* __restrict__ gv, WsHeader* hdr,
+__global__ void __launch_bounds__(kThreads) k_grid_pack_user(int64_t nn, const T* __restrict__ gv,
                                                              Node4<T>* __restrict__ B) {
   dep_wait();
   for (int64_t node = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; node < nn;
        node += (int64_t)gridDim.x * blockDim.x) {
     T v[3] = {gv[node * DIM + 0], gv[node * DIM + 1], T(0)};
     if constexpr (DIM == 3) v[2] = gv[node * DIM + 2];
-    if (nonfinite_probe(v, 3) != T(0)) hdr->b_dirty = 1u;
     B[node] = Node4<T>{v[0], v[1], v[2], T(0)};
   }
 }
