@@ -80,29 +80,12 @@ struct RunLane {
 
 // Sums of the records [l0, l1) of a list grouped by base node (stride kS reals, shared memory) in
 // registers while the base node stays the same, then one vector reduction per node into A.  The
-// bounds may differ from group to group.  Momenta are summed relative to a velocity u that the list has
-// about in common, sum w (q - m u + a o), and u sum w m is added at the end of a run: the part in common so
-// takes no rounding from the run's length.
+// bounds may differ from group to group.  The sums hold momenta as they are: taken relative to a velocity of the
+// list, one light or fast particle would cost every node of the list its digits.
 template <int DIM, typename T>
-__device__ __forceinline__ void run_add(Node4<T>* at, const T (&a)[4], const T (&u)[DIM]) {
-  atomic_add4(at, a[0] + u[0] * a[3], a[1] + u[1] * a[3], DIM == 3 ? a[2] + u[DIM - 1] * a[3] : T(0), a[3]);
-}
-template <int DIM, typename T>
-__device__ __forceinline__ void run_flush(Node4<T>* at, const T (&acc)[DIM == 3 ? 3 : 1][4], const T (&u)[DIM],
-                                          int64_t RR) {
+__device__ __forceinline__ void run_flush(Node4<T>* at, const T (&acc)[DIM == 3 ? 3 : 1][4], int64_t RR) {
 #pragma unroll
-  for (int i = 0; i < (DIM == 3 ? 3 : 1); ++i) run_add<DIM, T>(at + i * RR, acc[i], u);
-}
-
-// q / m of a record, or zero where that is no usable velocity.
-template <int DIM, typename T>
-__device__ __forceinline__ void run_velocity(const T* rec, T (&u)[DIM]) {
-  const T im = rec[0] > T(0) ? ffrcp(rec[0]) : T(0);
-#pragma unroll
-  for (int r = 0; r < DIM; ++r) {
-    const T ur = rec[1 + r] * im;
-    u[r] = ffabs(ur) < T(1e18) ? ur : T(0);
-  }
+  for (int i = 0; i < (DIM == 3 ? 3 : 1); ++i) atomic_add4(at + i * RR, acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
 }
 
 // A group's sums under way.
@@ -110,7 +93,7 @@ template <int DIM, typename T>
 struct RunSums {
   static constexpr int NX = RunLane<DIM, T>::NX;
   int cur = -1;  // base node of the run (none yet: negative)
-  T acc[NX][4] = {}, u[DIM] = {};
+  T acc[NX][4] = {};
   T tot[NX][4] = {};  // what acc held at the ends of the run's earlier stages: a long run is a sum of sums
   __device__ __forceinline__ void put_by() {
 #pragma unroll
@@ -132,10 +115,10 @@ struct RunSums {
   }
 };
 
-// kStages: the list is one of several that a run may go through (put_by between them), and its records hold
-// q; else they hold q - m u already.  kSlide: keep the sums of shared nodes from cell to cell, which leaves a
-// third of the reductions, so that a node is a sum of fewer parts; it costs 24 shuffles a cell (the
-// resident solver, 16,384 particles: 668 us a call with it, 613 without).
+// kStages: the list is one of several that a run may go through (put_by between them).  kSlide: keep the
+// sums of shared nodes from cell to cell, which leaves a third of the reductions, so that a node is a sum of
+// fewer parts; it costs 24 shuffles a cell (the resident solver, 16,384 particles: 668 us a call with it, 613
+// without).
 template <int DIM, typename T, int kS, bool kStages, bool kSlide>
 __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, const int* nodes, int l0, int l1,
                                          const RunLane<DIM, T>& ln, Node4<T>* __restrict__ Al, int64_t RR) {
@@ -161,7 +144,7 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
         const unsigned group = 0x1ffu << (9 * ln.grp);
 #pragma unroll
         for (int i = 0; i < NX; ++i) {
-          if (ln.ob == 0) run_add<DIM, T>(Al + rs.cur + i * RR, rs.acc[i], rs.u);
+          if (ln.ob == 0) atomic_add4(Al + rs.cur + i * RR, rs.acc[i][0], rs.acc[i][1], rs.acc[i][2], rs.acc[i][3]);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             const T t = __shfl_down_sync(group, rs.acc[i][r], 1);
@@ -169,15 +152,11 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
           }
         }
       } else {
-        if (rs.cur >= 0) run_flush<DIM, T>(Al + rs.cur, rs.acc, rs.u, RR);
+        if (rs.cur >= 0) run_flush<DIM, T>(Al + rs.cur, rs.acc, RR);
 #pragma unroll
         for (int i = 0; i < NX; ++i) rs.acc[i][0] = rs.acc[i][1] = rs.acc[i][2] = rs.acc[i][3] = T(0);
       }
       rs.cur = nd;
-    }
-    if constexpr (kStages) {
-#pragma unroll
-      for (int r = 0; r < DIM; ++r) rv[1 + r] -= rv[0] * rs.u[r];
     }
     if constexpr (DIM == 3) {
       const T da = rv[f0 + 1] - ln.ra, db = rv[f0 + 2] - ln.rb;
@@ -217,12 +196,6 @@ __device__ __forceinline__ void run_end(RunSums<DIM, T>& rs, const RunLane<DIM, 
   const int c0 = __shfl_sync(kFull, rs.cur, 0), c1 = __shfl_sync(kFull, rs.cur, 9), c2 = __shfl_sync(kFull, rs.cur, 18);
   if (c1 >= 0 && (c0 == c1 || c1 == c2)) {
 #pragma unroll
-    for (int i = 0; i < NX; ++i)
-#pragma unroll
-      for (int r = 0; r < DIM; ++r) rs.acc[i][r] += rs.u[r] * rs.acc[i][3];
-#pragma unroll
-    for (int r = 0; r < DIM; ++r) rs.u[r] = T(0);
-#pragma unroll
     for (int to = 1; to >= 0; --to) {
       const bool join = to == 1 ? c1 == c2 : c0 == c1;
 #pragma unroll
@@ -235,7 +208,7 @@ __device__ __forceinline__ void run_end(RunSums<DIM, T>& rs, const RunLane<DIM, 
       if (join && ln.grp == to + 1) rs.cur = -1;
     }
   }
-  if (rs.cur >= 0) run_flush<DIM, T>(Al + rs.cur, rs.acc, rs.u, RR);
+  if (rs.cur >= 0) run_flush<DIM, T>(Al + rs.cur, rs.acc, RR);
 }
 
 // Scatter of one warp's 32 particles.  Every lane hands in its particle's record (`node`: linear index
@@ -280,21 +253,12 @@ __device__ __forceinline__ int warp_group(WarpRecs<DIM, T>& wr, const T (&rec)[R
 }
 
 template <int DIM, typename T>
-__device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec_in)[RunRec<DIM>::kPacked], int node,
+__device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec)[RunRec<DIM>::kPacked], int node,
                                              const RunLane<DIM, T>& ln, Node4<T>* __restrict__ A, int R) {
   constexpr unsigned kFull = 0xffffffffu;
   const unsigned vmask = __ballot_sync(kFull, node >= 0);
   if (vmask == 0u) return;
   RunSums<DIM, T> rs;
-  run_velocity<DIM, T>(rec_in, rs.u);
-  T rec[RunRec<DIM>::kPacked];
-#pragma unroll
-  for (int i = 0; i < RunRec<DIM>::kPacked; ++i) rec[i] = rec_in[i];
-#pragma unroll
-  for (int r = 0; r < DIM; ++r) {
-    rs.u[r] = __shfl_sync(kFull, rs.u[r], __ffs(vmask) - 1);
-    rec[1 + r] -= rec[0] * rs.u[r];
-  }
   const int nv = warp_group<DIM, T>(wr, rec, node, vmask);
   const int per = (nv + 2) / 3;
   const int l0 = ln.grp * per;
@@ -532,7 +496,6 @@ __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ r
     fetch(k);
     __syncwarp();
     const int l0 = kPitch * min(ln.grp, 2);
-    if (k == 0 && my_len > 0) run_velocity<DIM, T>(ws.rec[l0], rs.u);
     run_sums<DIM, T, kS, true, true>(rs, &ws.rec[0][0], ws.node, l0, l0 + max(0, min(32, my_len - 32 * k)), ln, Al, RR);
     rs.put_by();
     __syncwarp();
