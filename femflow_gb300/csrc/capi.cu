@@ -483,6 +483,13 @@ void launch_g2p_sorted(const ffmpm_params& p, const Layout& L, const Ws& w, cons
                                                                  w.hdr, w.tmark, w.touched);
 }
 
+// Half of an SM for the stages of k_cell_sums.  With what fills the SM (13 CTAs, 229 KB) the kernels that follow
+// in the chain of dependent launches are left with the L1 of that split, and k_g2p_range takes twice its time:
+// 480,000 particles on 96^3, two substeps: 574 us, 406 like this and 407 with 30.  A corrected coarse step of
+// 1,048,576 particles, which launches its gather plainly: 532 us, 541 like this and 551 with 30; of 400,000 on 64^3:
+// 243, 230 and 227.
+constexpr int kSumsCarveout = 50;
+
 // Scatter of the whole state into grid A.  Particles that may lie in any order are put in cell order
 // first; double particles, small counts and particles that the caller keeps in cell order
 // (kVariantCellOrder) are scattered as they come.
@@ -502,7 +509,7 @@ void scatter_unsorted(const ffmpm_params& p, const Layout& L, const Ws& w, const
       launch(true, k_cell_records<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, rank, w.cell_start, recs, nodes, &w.hdr->status,
                                                      &w.hdr->polar_fallbacks);
       const size_t smem = 2 * sizeof(WarpStage<DIM, T>);
-      launch(true, k_cell_sums<DIM, T>, (unsigned)((L.n + 191) / 192), 64, smem, s, L.R, recs, nodes, w.hdr,
+      launch_carved(kSumsCarveout, true, k_cell_sums<DIM, T>, (unsigned)((L.n + 191) / 192), 64, smem, s, L.R, recs, nodes, w.hdr,
                                                                           static_cast<Node4<T>*>(w.gridA));
       return;
     }

@@ -30,19 +30,32 @@ __device__ __forceinline__ void dep_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// `carveout`: percentage of an SM's shared memory and L1 that this launch wants as shared memory (negative: what
+// fills the SM with its CTAs).
 template <typename... P, typename... A>
-inline void launch(bool dep, void (*kern)(P...), int64_t grid, int threads, size_t smem, cudaStream_t s, A&&... args) {
+inline void launch_carved(int carveout, bool dep, void (*kern)(P...), int64_t grid, int threads, size_t smem, cudaStream_t s,
+                          A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = dep ? 1 : 0;
+  if (dep) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (carveout >= 0) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[cfg.numAttrs++].val.sharedMemCarveout = (unsigned)carveout;
+  }
   cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+template <typename... P, typename... A>
+inline void launch(bool dep, void (*kern)(P...), int64_t grid, int threads, size_t smem, cudaStream_t s, A&&... args) {
+  launch_carved(-1, dep, kern, grid, threads, smem, s, args...);
 }
 
 // ----------------------------------------------------------------------------------------------

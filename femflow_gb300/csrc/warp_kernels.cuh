@@ -94,50 +94,69 @@ struct RunSums {
   static constexpr int NX = RunLane<DIM, T>::NX;
   int cur = -1;  // base node of the run (none yet: negative)
   T acc[NX][4] = {};
-  T tot[NX][4] = {};  // what acc held at the ends of the run's earlier stages: a long run is a sum of sums
-  __device__ __forceinline__ void put_by() {
-#pragma unroll
-    for (int i = 0; i < NX; ++i)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        tot[i][r] += acc[i][r];
-        acc[i][r] = T(0);
-      }
-  }
+  T kept[NX][4] = {};  // kSlide: what the cells before brought to the run's nodes (a sum of cells' sums)
   __device__ __forceinline__ void take_up() {
 #pragma unroll
     for (int i = 0; i < NX; ++i)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        acc[i][r] += tot[i][r];
-        tot[i][r] = T(0);
+        acc[i][r] += kept[i][r];
+        kept[i][r] = T(0);
       }
   }
 };
 
-// kStages: the list is one of several that a run may go through (put_by between them).  kSlide: keep the
-// sums of shared nodes from cell to cell, which leaves a third of the reductions, so that a node is a sum of
-// fewer parts; it costs 24 shuffles a cell (the resident solver, 16,384 particles: 668 us a call with it, 613
-// without).
-template <int DIM, typename T, int kS, bool kStages, bool kSlide>
+// One record's contribution to the lane's nodes.
+template <int DIM, typename T>
+__device__ __forceinline__ void run_add(T (&acc)[DIM == 3 ? 3 : 1][4], const T* rec, const RunLane<DIM, T>& ln) {
+  constexpr int a0 = 1 + DIM, f0 = 1 + DIM + DIM * DIM, NV = RunRec<DIM>::kPacked / 4;
+  T rv[4 * NV];
+  const Node4<T>* src = reinterpret_cast<const Node4<T>*>(rec);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const Node4<T> q4 = src[i];
+    rv[4 * i] = q4.x;
+    rv[4 * i + 1] = q4.y;
+    rv[4 * i + 2] = q4.z;
+    rv[4 * i + 3] = q4.w;
+  }
+  if constexpr (DIM == 3) {
+    const T da = rv[f0 + 1] - ln.ra, db = rv[f0 + 2] - ln.rb;
+    const T wjk = (ln.ka * da * da + ln.ea) * (ln.kb * db * db + ln.eb);
+    T wx[3];
+    bspline(rv[f0], wx);
+    T b[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      b[r] = rv[1 + r] + rv[a0 + 3 * r + 1] * T(ln.oa) + rv[a0 + 3 * r + 2] * T(ln.ob);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const T wt = wx[i] * wjk;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) acc[i][r] += wt * (b[r] + T(i) * rv[a0 + 3 * r]);
+      acc[i][3] += wt * rv[0];
+    }
+  } else {
+    const T da = rv[f0] - ln.ra, db = rv[f0 + 1] - ln.rb;
+    const T wt = (ln.ka * da * da + ln.ea) * (ln.kb * db * db + ln.eb);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      acc[0][r] += wt * (rv[1 + r] + rv[a0 + 2 * r] * T(ln.oa) + rv[a0 + 2 * r + 1] * T(ln.ob));
+    acc[0][3] += wt * rv[0];
+  }
+}
+
+// kSlide: keep the sums of shared nodes from cell to cell, which leaves a third of the reductions, so that a
+// node is a sum of fewer parts; it costs 24 shuffles a cell (the resident solver, 16,384 particles: 668 us a
+// call with it, 613 without).
+template <int DIM, typename T, int kS, bool kSlide>
 __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, const int* nodes, int l0, int l1,
                                          const RunLane<DIM, T>& ln, Node4<T>* __restrict__ Al, int64_t RR) {
   constexpr int NX = RunLane<DIM, T>::NX;
-  constexpr int a0 = 1 + DIM, f0 = 1 + DIM + DIM * DIM, NV = RunRec<DIM>::kPacked / 4;
   for (int l = l0; l < l1; ++l) {
     const int nd = nodes[l];
-    T rv[4 * NV];
-    const Node4<T>* src = reinterpret_cast<const Node4<T>*>(recs + (size_t)l * kS);
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const Node4<T> q4 = src[i];
-      rv[4 * i] = q4.x;
-      rv[4 * i + 1] = q4.y;
-      rv[4 * i + 2] = q4.z;
-      rv[4 * i + 3] = q4.w;
-    }
     if (nd != rs.cur) {
-      if constexpr (kStages) rs.take_up();
+      if constexpr (kSlide) rs.take_up();
       if (kSlide && nd == rs.cur + 1 && rs.cur >= 0) {
         // the next cell along the grid's last axis shares two thirds of the nodes: the sums move one
         // lane down, and only those that no lane holds any more go to the grid
@@ -148,40 +167,17 @@ __device__ __forceinline__ void run_sums(RunSums<DIM, T>& rs, const T* recs, con
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             const T t = __shfl_down_sync(group, rs.acc[i][r], 1);
-            rs.acc[i][r] = ln.ob < 2 ? t : T(0);
+            rs.kept[i][r] = ln.ob < 2 ? t : T(0);
           }
         }
-      } else {
-        if (rs.cur >= 0) run_flush<DIM, T>(Al + rs.cur, rs.acc, RR);
-#pragma unroll
-        for (int i = 0; i < NX; ++i) rs.acc[i][0] = rs.acc[i][1] = rs.acc[i][2] = rs.acc[i][3] = T(0);
+      } else if (rs.cur >= 0) {
+        run_flush<DIM, T>(Al + rs.cur, rs.acc, RR);
       }
+#pragma unroll
+      for (int i = 0; i < NX; ++i) rs.acc[i][0] = rs.acc[i][1] = rs.acc[i][2] = rs.acc[i][3] = T(0);
       rs.cur = nd;
     }
-    if constexpr (DIM == 3) {
-      const T da = rv[f0 + 1] - ln.ra, db = rv[f0 + 2] - ln.rb;
-      const T wjk = (ln.ka * da * da + ln.ea) * (ln.kb * db * db + ln.eb);
-      T wx[3];
-      bspline(rv[f0], wx);
-      T b[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-        b[r] = rv[1 + r] + rv[a0 + 3 * r + 1] * T(ln.oa) + rv[a0 + 3 * r + 2] * T(ln.ob);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const T wt = wx[i] * wjk;
-#pragma unroll
-        for (int r = 0; r < 3; ++r) rs.acc[i][r] += wt * (b[r] + T(i) * rv[a0 + 3 * r]);
-        rs.acc[i][3] += wt * rv[0];
-      }
-    } else {
-      const T da = rv[f0] - ln.ra, db = rv[f0 + 1] - ln.rb;
-      const T wt = (ln.ka * da * da + ln.ea) * (ln.kb * db * db + ln.eb);
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-        rs.acc[0][r] += wt * (rv[1 + r] + rv[a0 + 2 * r] * T(ln.oa) + rv[a0 + 2 * r + 1] * T(ln.ob));
-      rs.acc[0][3] += wt * rv[0];
-    }
+    run_add<DIM, T>(rs.acc, recs + (size_t)l * kS, ln);
   }
 }
 
@@ -264,8 +260,8 @@ __device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec
   const int l0 = ln.grp * per;
   const int64_t RR = DIM == 3 ? (int64_t)R * R : 0;
   Node4<T>* const Al = A + (ln.oa * R + ln.ob);
-  run_sums<DIM, T, RunRec<DIM>::kSmem, false, false>(rs, &wr.rec[0][0], wr.node, l0,
-                                                     ln.grp < 3 ? min(nv, l0 + per) : 0, ln, Al, RR);
+  run_sums<DIM, T, RunRec<DIM>::kSmem, false>(rs, &wr.rec[0][0], wr.node, l0,
+                                              ln.grp < 3 ? min(nv, l0 + per) : 0, ln, Al, RR);
   run_end<DIM, T>(rs, ln, Al, RR);
   __syncwarp();  // the records are rewritten by the warp's next particles
 }
@@ -422,11 +418,17 @@ __global__ void __launch_bounds__(kThreads, 3) k_cell_records(KParams<T> kp, int
     dst[i] = Node4<T>{rec[4 * i], rec[4 * i + 1], rec[4 * i + 2], rec[4 * i + 3]};
 }
 
-// Each group of lanes sums a stretch of 32 x `stages` consecutive records (the three groups of a warp
-// neighbouring ones), 32 at a time: the records come to shared memory by asynchronous copies, while the
-// SM's other warps sum theirs.  A run that crosses the end of a stretch belongs
-// to the stretch it begins in when it began within the last 32 records, up to 32 records past the end;
-// so a cell of up to 32 particles is one sum, and a node receives 27 sums (3D).
+// A warp sums a stretch of consecutive records, 96 at a time: they come to shared memory by asynchronous copies,
+// while the SM's other warps sum theirs.  A run that crosses the end of a stretch belongs to the stretch it
+// begins in when it began within the last 32 records, up to 32 records past the end.
+//   Cells of a few particles: each group of lanes takes a third of the 96 (a stretch each), and keeps the sums of
+// shared nodes from cell to cell along the last axis (run_sums).
+//   Fuller cells: a third would be one or two cells, and a node would receive nearly a part per cell, added in
+// no order.  So the groups share each run, add up what they have of it, and the warp goes from cell to cell with
+// the sums of shared nodes.  Float error of a corrected coarse step beside that of sums in block-sorted chunks
+// of 512: 0.97 times at 31 particles a cell (1,048,576 particles, 128^3), 1.07 at 24 (100,000, 64^3), 1.10 at 95
+// (400,000, 64^3), where thirds have 1.16, 1.24 and 1.29; as fast (541, 101 and 230 us, from 538, 103 and 238).
+// At 9 particles a cell it is slower (50,000 on 64^3: 93 us, 88 with thirds), for little (1.04, 1.09).
 template <int DIM, typename T>
 struct alignas(16) WarpStage {
   static constexpr int kPitch = 33;  // slots per group: the groups' reads fall on distinct banks
@@ -443,6 +445,8 @@ __device__ __forceinline__ int run_shift(const int* __restrict__ nodes, int at, 
   return !(after & 1u) && before ? (after ? __ffs(after) - 1 : 32) : 0;
 }
 
+constexpr int kFullCell = 14;  // particles a cell (mean) from which the groups share runs: two cells to a third
+
 template <int DIM, typename T>
 __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ recs, const int* __restrict__ nodes,
                                                   const WsHeader* hdr, Node4<T>* __restrict__ A) {
@@ -455,53 +459,90 @@ __global__ void __launch_bounds__(64) k_cell_sums(int R, const T* __restrict__ r
   const int lane = threadIdx.x & 31;
   const int total = (int)hdr->cell_cursor;
   if (total == 0) return;
-  // stretches of 32 while cells are smaller than that; longer ones for fuller cells, whose sums would
-  // otherwise reach the grid in many pieces
   const int mean = total / (int)max(1u, hdr->cell_occupied);
+  const bool full = mean >= kFullCell;
   const int stages = mean < 64 ? 1 : min(16, mean / 24);
   const int64_t s0 = (int64_t)(blockIdx.x * 2 + (threadIdx.x >> 5)) * 96 * stages;
   if (s0 >= total) return;
-  int lo[3], hi[3];
-#pragma unroll
-  for (int g = 0; g < 3; ++g) {
-    const int b = (int)min((int64_t)total, s0 + (int64_t)32 * stages * g);
-    lo[g] = b < total ? b + run_shift(nodes, b, total) : total;
-    if (g > 0) hi[g - 1] = lo[g];
-  }
-  {
-    const int b = (int)min((int64_t)total, s0 + (int64_t)96 * stages);
-    hi[2] = b < total ? b + run_shift(nodes, b, total) : total;
-  }
-  const int len = max(max(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
-  const int steps = (len + 31) / 32;
-  const auto fetch = [&](int k) {
-#pragma unroll
-    for (int g = 0; g < 3; ++g) {
-      const int b = lo[g] + 32 * k, nr = min(32, hi[g] - b);
-      for (int q = lane; q < nr * NV; q += 32) {
-        const int r = q / NV, c = q - r * NV;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&ws.rec[kPitch * g + r][4 * c])),
-                     "l"(recs + (size_t)(b + r) * RunRec<DIM>::kPacked + 4 * c)
-                     : "memory");
-      }
-      if (lane < nr) ws.node[kPitch * g + lane] = nodes[b + lane];
+  const auto stretch_at = [&](int64_t at) {
+    return at < total ? (int)at + run_shift(nodes, (int)at, total) : total;
+  };
+  // records [b, b + nr) to slots from `slot` on (every lane calls it)
+  const auto fetch = [&](int slot, int b, int nr) {
+    for (int q = lane; q < nr * NV; q += 32) {
+      const int r = q / NV, c = q - r * NV;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&ws.rec[slot + r][4 * c])),
+                   "l"(recs + (size_t)(b + r) * RunRec<DIM>::kPacked + 4 * c)
+                   : "memory");
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int r = lane; r < nr; r += 32) ws.node[slot + r] = nodes[b + r];
   };
   const int64_t RR = DIM == 3 ? (int64_t)R * R : 0;
   Node4<T>* const Al = A + (ln.oa * R + ln.ob);
-  const int my_len = ln.grp == 0 ? hi[0] - lo[0] : ln.grp == 1 ? hi[1] - lo[1] : ln.grp == 2 ? hi[2] - lo[2] : 0;
   RunSums<DIM, T> rs;
-  for (int k = 0; k < steps; ++k) {
-    fetch(k);
+  if (!full) {
+    const int lo[4] = {stretch_at(s0), stretch_at(s0 + 32), stretch_at(s0 + 64), stretch_at(s0 + 96)};
+    const int len = max(max(lo[1] - lo[0], lo[2] - lo[1]), lo[3] - lo[2]);
+    const int my_len = ln.grp == 0 ? lo[1] - lo[0] : ln.grp == 1 ? lo[2] - lo[1] : ln.grp == 2 ? lo[3] - lo[2] : 0;
+    for (int k = 0; k < len; k += 32) {
+#pragma unroll
+      for (int g = 0; g < 3; ++g) fetch(kPitch * g, lo[g] + k, min(32, lo[g + 1] - lo[g] - k));
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      const int l0 = kPitch * min(ln.grp, 2);
+      run_sums<DIM, T, kS, true>(rs, &ws.rec[0][0], ws.node, l0, l0 + max(0, min(32, my_len - k)), ln, Al, RR);
+      __syncwarp();
+    }
+    rs.take_up();
+    run_end<DIM, T>(rs, ln, Al, RR);
+    return;
+  }
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int NX = RunLane<DIM, T>::NX;
+  const int hi = stretch_at(s0 + 96 * stages);
+  for (int b = stretch_at(s0); b < hi; b += 96) {
+    const int nr = min(96, hi - b);
+    fetch(0, b, nr);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
-    const int l0 = kPitch * min(ln.grp, 2);
-    run_sums<DIM, T, kS, true, true>(rs, &ws.rec[0][0], ws.node, l0, l0 + max(0, min(32, my_len - 32 * k)), ln, Al, RR);
-    rs.put_by();
+    for (int l = 0; l < nr;) {
+      // the run's end: the first of the next 32 records with another node, if any
+      const int nd = ws.node[l];
+      int e = l;
+      unsigned other;
+      do {
+        const int i = e + lane;
+        other = __ballot_sync(kAll, i >= nr || ws.node[min(i, nr - 1)] != nd);
+        e += other ? __ffs(other) - 1 : 32;
+      } while (!other);
+      if (nd != rs.cur) {  // rs.acc: the first group's lanes hold the sums of the cells before
+        const bool next = nd == rs.cur + 1 && rs.cur >= 0;
+#pragma unroll
+        for (int i = 0; i < NX; ++i) {
+          if (ln.grp == 0 && rs.cur >= 0 && (!next || ln.ob == 0))
+            atomic_add4(Al + rs.cur + i * RR, rs.acc[i][0], rs.acc[i][1], rs.acc[i][2], rs.acc[i][3]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const T t = __shfl_down_sync(kAll, rs.acc[i][r], 1);
+            rs.acc[i][r] = next && ln.ob < 2 ? t : T(0);
+          }
+        }
+        rs.cur = nd;
+      }
+      T part[NX][4] = {};
+      const int per = (e - l + 2) / 3, l0 = l + ln.grp * per, l1 = ln.grp < 3 ? min(e, l0 + per) : 0;
+      for (int q = l0; q < l1; ++q) run_add<DIM, T>(part, &ws.rec[q][0], ln);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < NX; ++i)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          rs.acc[i][r] += part[i][r] + (__shfl_down_sync(kAll, part[i][r], 9) + __shfl_down_sync(kAll, part[i][r], 18));
+      l = e;
+    }
     __syncwarp();
   }
-  rs.take_up();
-  run_end<DIM, T>(rs, ln, Al, RR);
+  if (ln.grp == 0 && rs.cur >= 0) run_flush<DIM, T>(Al + rs.cur, rs.acc, RR);
 }
 
 // Grid update of every node (three_d/grid_op.py:5-47 / two_d/grid_op.py:5-24): momentum of A ->
