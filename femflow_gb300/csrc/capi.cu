@@ -71,15 +71,20 @@ bool unsorted(const ffmpm_params& p, const Layout& L) {
          L.nnodes <= std::max<int64_t>(int64_t(1) << 22, 16 * L.n);
 }
 
-// Whether such an operation's workspace has room for the counting sort by cell: float particles, and
-// more of them than are scattered as they come (kScatterMax).  Scattered in a random order a node
-// sums its particles one after another: at 30 particles a cell the float error of a substep's C was five
-// times that of sums over cells.  Up to 4096 particles that does not show (2,048 particles at 4 a cell:
-// the same error), and one launch does the work of four.
-constexpr int64_t kScatterMax = 4096;
-bool cell_sorted(const ffmpm_params& p, const Layout& L) {
-  return p.real_bytes == 4 && !p.deterministic && L.n > kScatterMax &&
-         L.nnodes <= std::max<int64_t>(int64_t(1) << 22, 16 * L.n);
+// How such an operation scatters particles that may lie in any order (warp_kernels.cuh).  As they come, a node
+// sums its particles one after another, and the float error of a substep's C grows, beside that of the block sort,
+// with the particles of a cell: 1.01 times for 2,048 in 3D at 4, 1.02 for 4,096 at 8, 1.04 for 2,000 in 2D at 6, 1.12
+// for 4,000 at 12, and 5 times for many at 30.  Small counts, whose cells hold few, are scattered so all the same:
+// one launch does the work of four (2,048 particles, eight substeps: 333 us, 416 in cell order).
+// Double particles, and no more float ones than kRecordsMin, are put in order as a permutation: records in cell
+// order (float64 ones of 128 bytes) take three times as long (200,000 in 2D, four substeps: 2,590 us, 917 as a
+// permutation and 1,154 as they come).
+enum class ScatterForm { kAsTheyCome, kPermuted, kRecords };
+constexpr int64_t kRecordsMin = 4096;
+ScatterForm scatter_form(const ffmpm_params& p, const Layout& L) {
+  if (p.deterministic || L.n <= (p.dim == 3 ? 4096 : 2048) || L.nnodes > std::max<int64_t>(int64_t(1) << 22, 16 * L.n))
+    return ScatterForm::kAsTheyCome;
+  return p.real_bytes == 8 || L.n <= kRecordsMin ? ScatterForm::kPermuted : ScatterForm::kRecords;
 }
 
 }  // namespace
@@ -135,12 +140,14 @@ bool make_layout(const ffmpm_params& p, int64_t n, Layout* L) {
   L->off_plan_cta = take(2 * 16 * ((L->nblocks + kPlanCta - 1) / kPlanCta));
   // the counting sort by cell of the unsorted operations (warp_kernels.cuh): counters and first slots
   // per node, and the records in cell order
-  if (cell_sorted(p, *L)) {
+  const ScatterForm form = scatter_form(p, *L);
+  if (form != ScatterForm::kAsTheyCome) {
     const size_t cells = align_up(size_t(L->nnodes), kCellTile);
     L->off_cell_count = take(sizeof(uint32_t) * cells);
     L->off_cell_start = take(sizeof(uint32_t) * cells);
-    L->off_recs = take(sizeof(float) * (p.dim == 3 ? RunRec<3>::kPacked : RunRec<2>::kPacked) * n);
   }
+  if (form == ScatterForm::kRecords)
+    L->off_recs = take(sizeof(float) * (p.dim == 3 ? RunRec<3>::kPacked : RunRec<2>::kPacked) * n);
   L->total = off;
   return true;
 }
@@ -462,11 +469,11 @@ struct WarpShape {
 
 template <int DIM, typename T>
 void launch_p2g_warp(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, const uint32_t* perm,
-                     int64_t p0, int64_t p1, cudaStream_t s, bool dep) {
+                     int64_t p0, int64_t p1, cudaStream_t s, bool dep, bool may_give_up = false) {
   const WarpShape<T> sh(p1 - p0, 8);
   const size_t smem = sizeof(WarpRecs<DIM, T>) * (sh.threads / 32);
-  launch(dep, k_p2g_warp<DIM, T>, sh.grid, sh.threads, smem, s, kparams<T>(p), geom<DIM>(L), P, perm, (uint32_t)p0,
-                                                       (uint32_t)p1, static_cast<Node4<T>*>(w.gridA), &w.hdr->status,
+  launch(dep, k_p2g_warp<DIM, T>, sh.grid, sh.threads, smem, s, kparams<T>(p), geom<DIM>(L), P, perm,
+                                                       may_give_up, (uint32_t)p0, (uint32_t)p1, static_cast<Node4<T>*>(w.gridA), &w.hdr->status,
                                                        &w.hdr->polar_fallbacks);
 }
 
@@ -491,30 +498,34 @@ void launch_g2p_sorted(const ffmpm_params& p, const Layout& L, const Ws& w, cons
 constexpr int kSumsCarveout = 50;
 
 // Scatter of the whole state into grid A.  Particles that may lie in any order are put in cell order
-// first; double particles, small counts and particles that the caller keeps in cell order
-// (kVariantCellOrder) are scattered as they come.
+// first (scatter_form), unless the caller keeps them so (kVariantCellOrder).
 template <int DIM, typename T>
 void scatter_unsorted(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, cudaStream_t s) {
-  if constexpr (sizeof(T) == 4) {
-    if (cell_sorted(p, L) && !(p.variant & kVariantCellOrder)) {
-      const KParams<T> kp = kparams<T>(p);
-      const uint32_t n = (uint32_t)L.n;
-      const unsigned pg = (n + kThreads - 1) / kThreads;
-      uint32_t* rank = w.keys0;
-      int* nodes = reinterpret_cast<int*>(w.vals0);
-      T* recs = static_cast<T*>(w.recs);
-      launch(false, k_cell_rank<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, w.cell_count, rank);
-      launch(true, k_cell_offsets, (unsigned)((L.nnodes + kCellTile - 1) / kCellTile), kThreads, 0, s, 
-          w.cell_count, w.cell_start, w.hdr);
-      launch(true, k_cell_records<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, rank, w.cell_start, recs, nodes, &w.hdr->status,
-                                                     &w.hdr->polar_fallbacks);
-      const size_t smem = 2 * sizeof(WarpStage<DIM, T>);
-      launch_carved(kSumsCarveout, true, k_cell_sums<DIM, T>, (unsigned)((L.n + 191) / 192), 64, smem, s, L.R, recs, nodes, w.hdr,
-                                                                          static_cast<Node4<T>*>(w.gridA));
-      return;
-    }
+  const ScatterForm form = p.variant & kVariantCellOrder ? ScatterForm::kAsTheyCome : scatter_form(p, L);
+  if (form == ScatterForm::kAsTheyCome) {
+    launch_p2g_warp<DIM, T>(p, L, w, P, nullptr, 0, L.n, s, false);
+    return;
   }
-  launch_p2g_warp<DIM, T>(p, L, w, P, nullptr, 0, L.n, s, false);
+  const KParams<T> kp = kparams<T>(p);
+  const uint32_t n = (uint32_t)L.n;
+  const unsigned pg = (n + kThreads - 1) / kThreads;
+  uint32_t* rank = w.keys0;
+  int* nodes = reinterpret_cast<int*>(w.vals0);  // by particle (kPermuted) or by slot (kRecords)
+  const bool permuted = form == ScatterForm::kPermuted;
+  launch(false, k_cell_rank<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, w.cell_count, rank, permuted ? nodes : nullptr);
+  launch(true, k_cell_offsets, (L.nnodes + kCellTile - 1) / kCellTile, kThreads, 0, s, w.cell_count, w.cell_start, w.hdr);
+  if (permuted) {
+    launch(true, k_cell_perm, pg, kThreads, 0, s, n, rank, nodes, w.cell_start, w.hdr, w.keys1);
+    launch_p2g_warp<DIM, T>(p, L, w, P, w.keys1, 0, L.n, s, true);
+    return;
+  }
+  if constexpr (sizeof(T) == 4) {
+    T* recs = static_cast<T*>(w.recs);
+    launch(true, k_cell_records<DIM, T>, pg, kThreads, 0, s, kp, L.R, P, n, rank, w.cell_start, recs, nodes, &w.hdr->status,
+           &w.hdr->polar_fallbacks);
+    launch_carved(kSumsCarveout, true, k_cell_sums<DIM, T>, (L.n + 191) / 192, 64, 2 * sizeof(WarpStage<DIM, T>), s, L.R,
+                  recs, nodes, w.hdr, static_cast<Node4<T>*>(w.gridA));
+  }
 }
 
 template <int DIM, typename T>
@@ -719,7 +730,7 @@ int op_substeps_fused(const ffmpm_params& p, const Layout& L, const Ws& w, PView
   sort_and_plan<DIM, T>(p, L, w, va, false, &sorted_perm, s, tm, nullptr, 1);
   const uint32_t* perm = sorted_perm;  // the permutation the next P2G / G2P applies (null: none)
   if (tm) tm->begin(3);
-  launch_p2g_warp<DIM, T>(p, L, w, va, perm, 0, L.n, s, true);
+  launch_p2g_warp<DIM, T>(p, L, w, va, perm, 0, L.n, s, true, true);
   if (tm) tm->end(1);
   for (int k = 0; k < nsteps; ++k) {
     const PView<T>& in = (k & 1) ? vb : va;

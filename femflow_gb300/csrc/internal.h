@@ -27,7 +27,8 @@ struct WsHeader {
   uint32_t det_next[2];  // deterministic P2G: next entry of the occupied list, per pass (zeroed per launch)
   uint32_t cell_cursor;  // slots handed out by k_cell_offsets (zeroed by the grid pass that follows)
   uint32_t cell_occupied;  // cells with particles, as counted by k_cell_offsets (zeroed with it)
-  uint32_t pad[52];
+  uint32_t cell_outside;  // particles outside the grid, as counted by k_cell_perm (zeroed with it)
+  uint32_t pad[51];
 };
 static_assert(sizeof(WsHeader) == 256, "header is one 256-byte line");
 

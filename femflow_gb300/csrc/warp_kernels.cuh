@@ -271,14 +271,15 @@ __device__ __forceinline__ void warp_scatter(WarpRecs<DIM, T>& wr, const T (&rec
 template <typename T>
 constexpr int kWarpCta = sizeof(T) == 4 ? 256 : 128;
 
-// P2G of particles [p0, p1) (through perm, when given) into the workspace grid A.
+// P2G of particles [p0, p1) (through perm, when given) into the workspace grid A.  `may_give_up`: perm comes from
+// the radix sort, whose bounded wait may have left it incomplete.
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom<DIM> g, PView<T> P,
-                                                            const uint32_t* __restrict__ perm, uint32_t p0,
-                                                            uint32_t p1, Node4<T>* __restrict__ A, int32_t* status,
-                                                            uint32_t* fallbacks) {
+                                                            const uint32_t* __restrict__ perm, bool may_give_up,
+                                                            uint32_t p0, uint32_t p1, Node4<T>* __restrict__ A,
+                                                            int32_t* status, uint32_t* fallbacks) {
   dep_wait();
-  if (perm && wait_gave_up(status)) return;
+  if (may_give_up && wait_gave_up(status)) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   WarpRecs<DIM, T>& wr = reinterpret_cast<WarpRecs<DIM, T>*>(smem_raw)[threadIdx.x >> 5];
   const RunLane<DIM, T> ln;
@@ -297,14 +298,17 @@ __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom
 }
 
 // ----------------------------------------------------------------------------------------------
-// Float particles in no order: a node then receives hundreds of contributions one at a time, and the
-// float sum loses what a sum over cells keeps.  So the records are put in cell order first, by a
-// counting sort whose counters are the grid's nodes:
+// Particles in no order: a node then receives hundreds of contributions one at a time, and the sum loses what
+// a sum over cells keeps.  So they are put in cell order first, by a counting sort whose counters are the grid's
+// nodes:
 //   k_cell_rank     each particle's rank among those of its base node (one atomic per warp and node)
 //   k_cell_offsets  first slot of every occupied node: tiles of nodes take their slots from one
 //                   counter, so the tiles may come in any order and no CTA waits on another
 //   k_cell_records  stress and record of every particle, written to its slot
 //   k_cell_sums     run sums over the records as they lie
+// or, for double particles and few float ones, whose records cost more to write and to wait for than their
+// particles to gather:
+//   k_cell_perm     the particles' indices in their slots, for k_p2g_warp
 // 1,048,576 particles of a random order on 128^3, component-major (GB300): 18 + 5 + 79 + 50 us, where
 // the block sort and the chunked scatter through its permutation took 150 + 305 us (every component
 // of a particle then came from a sector of its own).  k_cell_records is bound by its scattered 64-byte
@@ -327,7 +331,8 @@ __device__ __forceinline__ int base_node(const KParams<T>& kp, const PView<T>& P
 
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_cell_rank(KParams<T> kp, int R, PView<T> P, uint32_t n,
-                                                        uint32_t* __restrict__ count, uint32_t* __restrict__ rank) {
+                                                        uint32_t* __restrict__ count, uint32_t* __restrict__ rank,
+                                                        int* __restrict__ node_of) {
   dep_wait();
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   const int node = p < n ? base_node<DIM, T>(kp, P, p, R) : -1;
@@ -336,7 +341,10 @@ __global__ void __launch_bounds__(kThreads) k_cell_rank(KParams<T> kp, int R, PV
   uint32_t first = 0;
   if (node >= 0 && before == 0u) first = atomicAdd(&count[node], (uint32_t)__popc(peers));
   first = __shfl_sync(0xffffffffu, first, __ffs(peers) - 1);
-  if (p < n) rank[p] = node >= 0 ? first + __popc(before) : kNoRank;
+  if (p < n) {
+    rank[p] = node >= 0 ? first + __popc(before) : kNoRank;
+    if (node_of) node_of[p] = node;
+  }
 }
 
 // count -> start (occupied nodes only); the counters go back to zero for the next call.
@@ -418,6 +426,18 @@ __global__ void __launch_bounds__(kThreads, 3) k_cell_records(KParams<T> kp, int
     dst[i] = Node4<T>{rec[4 * i], rec[4 * i + 1], rec[4 * i + 2], rec[4 * i + 3]};
 }
 
+// The particles in cell order as a permutation; those outside the grid, which no cell counted, come last.
+static __global__ void __launch_bounds__(kThreads) k_cell_perm(uint32_t n, const uint32_t* __restrict__ rank,
+                                                               const int* __restrict__ node_of,
+                                                               const uint32_t* __restrict__ start, WsHeader* hdr,
+                                                               uint32_t* __restrict__ perm) {
+  dep_wait();
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int node = node_of[p];
+  perm[node >= 0 ? start[node] + rank[p] : hdr->cell_cursor + atomicAdd(&hdr->cell_outside, 1u)] = p;
+}
+
 // A warp sums a stretch of consecutive records, 96 at a time: they come to shared memory by asynchronous copies,
 // while the SM's other warps sum theirs.  A run that crosses the end of a stretch belongs to the stretch it
 // begins in when it began within the last 32 records, up to 32 records past the end.
@@ -427,7 +447,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_cell_records(KParams<T> kp, int
 // no order.  So the groups share each run, add up what they have of it, and the warp goes from cell to cell with
 // the sums of shared nodes.  Float error of a corrected coarse step beside that of sums in block-sorted chunks
 // of 512: 0.97 times at 31 particles a cell (1,048,576 particles, 128^3), 1.07 at 24 (100,000, 64^3), 1.10 at 95
-// (400,000, 64^3), where thirds have 1.16, 1.24 and 1.29; as fast (541, 101 and 230 us, from 538, 103 and 238).
+// (400,000, 64^3), where thirds have 1.16, 1.24 and 1.32; as fast (541, 101 and 230 us, from 538, 103 and 238).
 // At 9 particles a cell it is slower (50,000 on 64^3: 93 us, 88 with thirds), for little (1.04, 1.09).
 template <int DIM, typename T>
 struct alignas(16) WarpStage {
@@ -556,7 +576,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_update_dense(KParams<T> kp, G
   dep_wait();
   const int R = g.R;
   const int64_t nn = DIM == 3 ? (int64_t)R * R * R : (int64_t)R * R;
-  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = 0u;  // for the next call's k_cell_offsets
+  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = hdr->cell_outside = 0u;  // for the next call
   constexpr int U = 4;  // nodes of a thread in flight
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t n0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n0 < nn; n0 += U * stride) {
@@ -694,7 +714,7 @@ template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_fold_user(int64_t nn, WsHeader* hdr, Node4<T>* __restrict__ A, T* __restrict__ gv,
                                                              T* __restrict__ gm) {
   dep_wait();
-  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = 0u;  // for the next call's k_cell_offsets
+  if (blockIdx.x == 0 && threadIdx.x == 0) hdr->cell_cursor = hdr->cell_occupied = hdr->cell_outside = 0u;  // for the next call
   for (int64_t node = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; node < nn;
        node += (int64_t)gridDim.x * blockDim.x) {
     const Node4<T> a = A[node];
