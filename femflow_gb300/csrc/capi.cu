@@ -9,10 +9,10 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <set>
 #include <vector>
 
 #include "common.cuh"
+#include "device_once.h"
 #include "internal.h"
 #include "mpm_kernels.cuh"
 #include "warp_kernels.cuh"
@@ -150,6 +150,17 @@ bool make_layout(const ffmpm_params& p, int64_t n, Layout* L) {
     L->off_recs = take(sizeof(float) * (p.dim == 3 ? RunRec<3>::kPacked : RunRec<2>::kPacked) * n);
   L->total = off;
   return true;
+}
+
+bool allow_smem(const void* kernel, size_t bytes) {
+  static DeviceOnce once;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return once.run(dev, kernel, [&] {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+  });
 }
 
 int sm_count() {
@@ -371,16 +382,9 @@ size_t cells_smem_bytes(const Layout& L) {
                     : tile_smem<2, double>(L) + cell_run_smem_bytes<2, double>(L.bs);
 }
 
-// Raise a kernel's dynamic shared-memory limit once per kernel (a host-side attribute call,
-// kept out of CUDA-graph captures, which run after the first direct call).
 template <typename F>
 void set_smem(F* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return;
-  static std::mutex mu;
-  static std::set<const void*> done;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done.insert(reinterpret_cast<const void*>(kernel)).second)
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+  if (bytes > 48 * 1024) allow_smem(reinterpret_cast<const void*>(kernel), kMaxDynSmem);
 }
 
 template <int DIM, typename T, typename Sink>

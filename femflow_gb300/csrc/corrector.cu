@@ -485,11 +485,7 @@ int launch_corrector(const ffmpm_params& p, const ffmpm_grid& g, ffmpm_particles
                      uint16_t* feat, int* det_keys, int32_t* status, cudaStream_t s) {
   auto kern = k_corrector<A, E>;
   const size_t smem = SmemLayout::total;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
+  if (!allow_smem(reinterpret_cast<const void*>(kern), smem)) return FFMPM_ERR_CUDA;
   const int64_t tiles = (Pp.n + 127) / 128;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count()));
   ffmpm_mlp nn{};

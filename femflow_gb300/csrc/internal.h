@@ -42,6 +42,10 @@ struct Layout {
          off_hist = 0, off_gridA = 0, off_gridB = 0, off_stage = 0, off_plan_pref = 0, off_plan_cta = 0, off_cell_count = 0, off_cell_start = 0, off_recs = 0, total = 0;
 };
 
+// Raises the kernel's limit of dynamic shared memory on the current device to `bytes`, once (a host-side attribute
+// call, kept out of CUDA-graph captures, which run after the first direct call).  False: the device refuses.
+bool allow_smem(const void* kernel, size_t bytes);
+
 bool make_layout(const ffmpm_params& p, int64_t n, Layout* L);
 
 int sm_count();

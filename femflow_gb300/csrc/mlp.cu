@@ -121,11 +121,7 @@ template <int BN>
 int launch_gemm(const uint16_t* A, const uint16_t* B, float* D, int M, int N, int K, int split, int32_t* status,
                 cudaStream_t s) {
   const size_t smem = size_t(128 + BN) * kKChunk * 2;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_tc_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
+  if (!allow_smem(reinterpret_cast<const void*>(k_tc_gemm<BN>), smem)) return FFMPM_ERR_CUDA;
   const int chunks = K / kKChunk;
   split = std::max(1, std::min(split, chunks));
   const int per = (chunks + split - 1) / split * kKChunk;
@@ -553,14 +549,6 @@ bool aligned16(const ffmpm_mlp_trainer& t) {
            reinterpret_cast<uintptr_t>(t.Y) | reinterpret_cast<uintptr_t>(t.grads)) & 15) == 0;
 }
 
-// Raise a kernel's dynamic shared-memory limit (once: `done`).
-template <typename F>
-void allow_smem(F* kern, size_t bytes, bool* done) {
-  if (*done) return;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  *done = true;
-}
-
 }  // namespace
 }  // namespace ffmpm
 
@@ -584,8 +572,7 @@ int ffmpm_tc_gemm_bf16(const uint16_t* A, const uint16_t* B, float* D, int32_t M
 
 int ffmpm_mlp_train_forward(const ffmpm_mlp_trainer* t, const uint16_t* X, int32_t B, void* stream) {
   if (!t || !X || B <= 0 || B % 128 || B > t->max_batch || (reinterpret_cast<uintptr_t>(X) & 15)) return FFMPM_ERR_BADARG;
-  static bool allowed = false;
-  allow_smem(k_mlp_forward, FwdSmem::total, &allowed);
+  if (!allow_smem(reinterpret_cast<const void*>(k_mlp_forward), FwdSmem::total)) return FFMPM_ERR_CUDA;
   k_mlp_forward<<<B / 128, kTrain, FwdSmem::total, static_cast<cudaStream_t>(stream)>>>(*t, X, B, aligned16(*t));
   return cudaGetLastError() == cudaSuccess ? FFMPM_OK : FFMPM_ERR_CUDA;
 }
@@ -594,8 +581,7 @@ int ffmpm_mlp_train_backward(const ffmpm_mlp_trainer* t, const float* T, const f
                              void* stream) {
   if (!t || !T || !w || !loss || B <= 0 || B % 128 || B > t->max_batch) return FFMPM_ERR_BADARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  static bool allowed = false;
-  allow_smem(k_mlp_backward, BwdSmem::total, &allowed);
+  if (!allow_smem(reinterpret_cast<const void*>(k_mlp_backward), BwdSmem::total)) return FFMPM_ERR_CUDA;
   cudaMemsetAsync(t->grads, 0, sizeof(float) * FFMPM_MLP_PARAMS, s);
   k_mlp_backward<<<std::min(B / 128, sm_count()), kTrain, BwdSmem::total, s>>>(*t, T, w, B, loss, aligned16(*t));
   return cudaGetLastError() == cudaSuccess ? FFMPM_OK : FFMPM_ERR_CUDA;
