@@ -955,18 +955,26 @@ int prologue(const ffmpm_params* p, int64_t n, void* ws, size_t ws_bytes, Layout
 struct StatusSlot {
   uint32_t* p = nullptr;
   StatusSlot() {
-    // a thread's first read may fall into another thread's stream capture, which page-locking would spoil
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    const RelaxedCapture mode;
     if (cudaHostAlloc(reinterpret_cast<void**>(&p), 8, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
     }
-    cudaThreadExchangeStreamCaptureMode(&mode);
   }
   ~StatusSlot() {
-    if (p) cudaFreeHost(p);
+    if (!p) return;
+    const RelaxedCapture mode;
+    cudaFreeHost(p);
   }
+
+ private:
+  // a thread's first read, and its end, may fall into another thread's stream capture, which page-locking and its
+  // undoing would spoil
+  struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  };
 };
 uint32_t* status_slot() {
   static thread_local StatusSlot slot;
