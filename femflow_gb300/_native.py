@@ -52,7 +52,9 @@ class Params(ctypes.Structure):
 
 
 MAX_PLANES = 8
-VARIANT_CELL_ORDER = 16  # ffmpm_params.variant bit 4
+# ffmpm_params.variant bit 4: the in-place operations need not order the particles first (a hint; a workspace
+# made with it has no room for that)
+VARIANT_CELL_ORDER = 16
 PLANE_RULES = {"sticky": 0, "reference_literal": 1}
 
 

@@ -71,18 +71,20 @@ bool unsorted(const ffmpm_params& p, const Layout& L) {
          L.nnodes <= std::max<int64_t>(int64_t(1) << 22, 16 * L.n);
 }
 
-// How such an operation scatters particles that may lie in any order (warp_kernels.cuh).  As they come, a node
-// sums its particles one after another, and the float error of a substep's C grows, beside that of the block sort,
-// with the particles of a cell: 1.01 times for 2,048 in 3D at 4, 1.02 for 4,096 at 8, 1.04 for 2,000 in 2D at 6, 1.12
-// for 4,000 at 12, and 5 times for many at 30.  Small counts, whose cells hold few, are scattered so all the same:
-// one launch does the work of four (2,048 particles, eight substeps: 333 us, 416 in cell order).
+// How such an operation scatters particles that may lie in any order (warp_kernels.cuh), unless the caller keeps
+// them near cell order (kVariantCellOrder).  As they come, a node sums its particles one after another, and the float
+// error of a substep's C grows, beside that of the block sort, with the particles of a cell: 1.01 times for 2,048 in
+// 3D at 4, 1.02 for 4,096 at 8, 1.04 for 2,000 in 2D at 6, 1.12 for 4,000 at 12, and 5 times for many at 30.  Small
+// counts, whose cells hold few, are scattered so all the same: one launch does the work of four (2,048 particles,
+// eight substeps: 333 us, 416 in cell order).
 // Double particles, and no more float ones than kRecordsMin, are put in order as a permutation: records in cell
 // order (float64 ones of 128 bytes) take three times as long (200,000 in 2D, four substeps: 2,590 us, 917 as a
 // permutation and 1,154 as they come).
 enum class ScatterForm { kAsTheyCome, kPermuted, kRecords };
 constexpr int64_t kRecordsMin = 4096;
 ScatterForm scatter_form(const ffmpm_params& p, const Layout& L) {
-  if (p.deterministic || L.n <= (p.dim == 3 ? 4096 : 2048) || L.nnodes > std::max<int64_t>(int64_t(1) << 22, 16 * L.n))
+  if (p.deterministic || (p.variant & kVariantCellOrder) || L.n <= (p.dim == 3 ? 4096 : 2048) ||
+      L.nnodes > std::max<int64_t>(int64_t(1) << 22, 16 * L.n))
     return ScatterForm::kAsTheyCome;
   return p.real_bytes == 8 || L.n <= kRecordsMin ? ScatterForm::kPermuted : ScatterForm::kRecords;
 }
@@ -501,11 +503,10 @@ void launch_g2p_sorted(const ffmpm_params& p, const Layout& L, const Ws& w, cons
 // 243, 230 and 227.
 constexpr int kSumsCarveout = 50;
 
-// Scatter of the whole state into grid A.  Particles that may lie in any order are put in cell order
-// first (scatter_form), unless the caller keeps them so (kVariantCellOrder).
+// Scatter of the whole state into grid A, in the form that scatter_form names.
 template <int DIM, typename T>
 void scatter_unsorted(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<T>& P, cudaStream_t s) {
-  const ScatterForm form = p.variant & kVariantCellOrder ? ScatterForm::kAsTheyCome : scatter_form(p, L);
+  const ScatterForm form = scatter_form(p, L);
   if (form == ScatterForm::kAsTheyCome) {
     launch_p2g_warp<DIM, T>(p, L, w, P, nullptr, 0, L.n, s, false);
     return;

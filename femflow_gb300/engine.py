@@ -121,7 +121,8 @@ def status_message(st: int) -> str:
 
 def workspace_for(params: N.Params, n: int, device) -> Workspace:
     """Workspace cache keyed by the shape-determining parameters."""
-    key = (params.dim, params.res, params.real_bytes, params.deterministic, params.block_size, int(n),
+    key = (params.dim, params.res, params.real_bytes, params.deterministic, params.block_size,
+           params.variant & N.VARIANT_CELL_ORDER, int(n),
            torch.device(device).index)
     ws = _WS_CACHE.get(key)
     if ws is None:

@@ -74,7 +74,8 @@ class MPMSolver:
                                     0.0 if per_particle else float(mass), 0.0 if per_particle else float(mu_0),
                                     0.0 if per_particle else float(lambda_0), model=model, wall_mode=wall_mode,
                                     block_size=block_size,
-                                    variant=(variant & 0xFF) | (max(1, min(255, int(sort_every))) << 8),
+                                    # the state is in block order; nothing here orders it by cell
+                                    variant=(variant & 0xFF) | N.VARIANT_CELL_ORDER | (max(1, min(255, int(sort_every))) << 8),
                                     deterministic=deterministic, planes=planes, plane_rule=plane_rule)
         self._a = _Buffers(n, dim, dtype, device, per_particle)
         self._b = _Buffers(n, dim, dtype, device, per_particle)

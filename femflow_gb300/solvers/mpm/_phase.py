@@ -70,6 +70,8 @@ def run_host_substep(params: N.Params, x, mass, mu_0, lambda_0, v, F, C, Jp, che
     """One substep on pinned host arrays through ffmpm_substep_host (copies pipelined with the
     kernels), in place; returns once the host arrays hold the result."""
     device = torch.device(device or "cuda")
+    params = N.Params.from_buffer_copy(params)
+    params.variant |= N.VARIANT_CELL_ORDER  # chunks are scattered as they land: no room to order them by cell
     host = E.particles_struct(x, v, F, C, Jp, mass, mu_0, lambda_0)
     dx, dv, dF, dC, dJ, dm, dmu, dlam = _device_mirror([x, v, F, C, Jp, mass, mu_0, lambda_0], device)
     dev = E.particles_struct(dx, dv, dF, dC, dJ, dm, dmu, dlam)

@@ -88,7 +88,8 @@ typedef struct ffmpm_params {
                          * and P2G separately instead of the fused kernel; bit 4: the caller keeps its
                          * particles in about the order of their base cells, so that the in-place
                          * operations (ffmpm_substep, ffmpm_p2g) need not order them first (a hint: any
-                         * order is handled); bits 8..15: substeps between re-sorts of ffmpm_substeps_sorted (0 or 1: every substep) */
+                         * order is handled; a workspace sized with it has no room to order them and serves
+                         * calls with it); bits 8..15: substeps between re-sorts of ffmpm_substeps_sorted (0 or 1: every substep) */
   double dx, inv_dx, dt;
   double gravity;       /* added to the axis-1 (y) grid velocity, as the reference */
   double volume;        /* particle volume (reference argument `volume`) */
