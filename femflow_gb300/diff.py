@@ -22,7 +22,7 @@ Gradients with respect to Young's modulus and Poisson's ratio follow by autograd
 from __future__ import annotations
 
 import ctypes
-from dataclasses import dataclass, replace
+from dataclasses import dataclass
 
 import torch
 
@@ -45,7 +45,9 @@ class RolloutConfig:
     # planar colliders ((point, normal) pairs) applied by every grid update, and their rule
     planes: tuple = ()
     plane_rule: str = "sticky"
-    # the particles come in (about) the order of their base cells: ``simulate`` sets it when it orders them
+    # the particles are, and stay for all the steps, near the order of their base cells: the substeps do not order
+    # them first.  Sums then lose digits as particles move (two bodies of 30 particles a cell that have moved 0.8
+    # cells: v and C 1.5 times as far from 64 bits; of 120 a cell, 2.9 times)
     cell_order: bool = False
 
 
@@ -222,7 +224,8 @@ def simulate(x0, v0, mu_0, lambda_0, cfg: RolloutConfig, mass, F0=None, C0=None,
     F0, C0 default to the reference's initial state (identity, zero; mls_mpm.py:9-15).
     With ``order`` the rollout runs on the particles ordered by base cell (neighbouring lanes of the
     adjoint kernels then share stencil nodes); inputs and outputs stay in the caller's order, and
-    the rollout's state is gathered once each way.
+    the rollout's state is gathered once each way.  Particles move on from that order, so every substep puts
+    its scatter in cell order by itself.
     """
     n, d = x0.shape[0], x0.shape[1]
     dtype, dev = x0.dtype, x0.device
@@ -237,5 +240,4 @@ def simulate(x0, v0, mu_0, lambda_0, cfg: RolloutConfig, mass, F0=None, C0=None,
     perm = cell_order(x0, cfg.res)
     inv = torch.empty_like(perm)
     inv[perm] = torch.arange(n, device=perm.device)
-    cfg = replace(cfg, cell_order=True)
     return MPMRollout.apply(x0, v0, F0, C0, mu, lam, mass, cfg, perm, inv)
