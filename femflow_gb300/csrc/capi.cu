@@ -574,8 +574,9 @@ int op_substep(const ffmpm_params& p, const Layout& L, const Ws& w, ffmpm_partic
 // ----------------------------------------------------------------------------- host-array substep
 // Copy streams and events of ffmpm_substep_host, one set per device, created by the first call on
 // that device (with it current) and kept until the process exits.
-// 1,048,576 particles: 1,303 us a call with 5 chunks, 1,318 with 4, 1,356 with 6 (smaller copies)
-constexpr int kHostChunks = 5;
+// Four chunks: a fifth costs its copies and launches and hides less than that below a million particles
+// (262,145: 442 us, 463 with five; 400,000: 576, 601; 800,000: 1,001, 1,031; 1,048,576: 1,322, 1,310).
+constexpr int kHostChunks = 4;
 struct HostPipe {
   cudaStream_t up = nullptr, down = nullptr;
   cudaEvent_t start = nullptr, gathered_all = nullptr, down_done = nullptr;
