@@ -709,7 +709,8 @@ __global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 2 : 1) k_g2p_sor
 }
 
 // The sums of A (momentum xyz, mass) added into a caller's grid_velocity [nodes][DIM] and grid_mass
-// [nodes]; A re-zeroed.
+// [nodes]; A re-zeroed.  Atomically, as the block-sorted form adds: another stream may add other particles
+// (over another workspace) to the same grid.
 template <int DIM, typename T>
 __global__ void __launch_bounds__(kThreads) k_grid_fold_user(int64_t nn, WsHeader* hdr, Node4<T>* __restrict__ A, T* __restrict__ gv,
                                                              T* __restrict__ gm) {
@@ -719,10 +720,10 @@ __global__ void __launch_bounds__(kThreads) k_grid_fold_user(int64_t nn, WsHeade
        node += (int64_t)gridDim.x * blockDim.x) {
     const Node4<T> a = A[node];
     if (a.x == T(0) && a.y == T(0) && a.z == T(0) && a.w == T(0)) continue;
-    gv[node * DIM + 0] += a.x;
-    gv[node * DIM + 1] += a.y;
-    if constexpr (DIM == 3) gv[node * DIM + 2] += a.z;
-    gm[node] += a.w;
+    atomicAdd(&gv[node * DIM + 0], a.x);
+    atomicAdd(&gv[node * DIM + 1], a.y);
+    if constexpr (DIM == 3) atomicAdd(&gv[node * DIM + 2], a.z);
+    atomicAdd(&gm[node], a.w);
     A[node] = Node4<T>{T(0), T(0), T(0), T(0)};
   }
 }
