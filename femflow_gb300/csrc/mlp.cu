@@ -132,7 +132,7 @@ int launch_gemm(const uint16_t* A, const uint16_t* B, float* D, int M, int N, in
 }
 
 // ---------------------------------------------------------------------------------------------
-// Training: elementwise kernels between the GEMMs.
+// Training: the activation, its derivative, and the launch shape of the elementwise kernels (Adam, packing).
 constexpr int kEw = 256;
 
 __device__ __forceinline__ float gelu_f(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
@@ -215,7 +215,7 @@ struct FwdSmem {
 };
 
 // Y = network(X) (before out_scale, without b4).  Keeps Z1..Z3 (with the biases), H1..H3 = gelu(Z) and the
-// transposes Ht and Xt, as the ABI documents; the backward pass reads X, Z and H.  One CTA per 128 rows:
+// transposes Ht and Xt, as the ABI documents; the backward pass reads Y, Z and the transposes.  One CTA per 128 rows:
 // the layers follow one another in shared and tensor memory (an MMA a layer), so that X is read once and
 // everything is written once.
 __global__ void __launch_bounds__(kTrain) k_mlp_forward(ffmpm_mlp_trainer t, const uint16_t* __restrict__ X, int B,

@@ -68,11 +68,10 @@ class Net:
         self.out_scale = torch.ones(16, **f32)
         B = max_batch
         self.buf = dict(Z1=torch.zeros(B, 64, **f32), Z2=torch.zeros(B, 64, **f32), Z3=torch.zeros(B, 64, **f32),
-                        Y=torch.zeros(B, 16, **f32), dH=torch.zeros(B, 64, **f32),
+                        Y=torch.zeros(B, 16, **f32),
                         H1=torch.zeros(B, 64, **bf), H2=torch.zeros(B, 64, **bf), H3=torch.zeros(B, 64, **bf),
                         H1t=torch.zeros(64, B, **bf), H2t=torch.zeros(64, B, **bf), H3t=torch.zeros(64, B, **bf),
-                        Xt=torch.zeros(128, B, **bf), dY=torch.zeros(B, 64, **bf), dZ=torch.zeros(B, 64, **bf),
-                        dYt=torch.zeros(128, B, **bf), dZt=torch.zeros(128, B, **bf))
+                        Xt=torch.zeros(128, B, **bf))
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         self.step = 0
         self.repack()
