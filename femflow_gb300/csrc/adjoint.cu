@@ -4,7 +4,7 @@
 //
 // The substep is x, v, F, C -> P2G -> grid update -> G2P -> x', v', F', C'.  Its reverse, given the
 // adjoints of x', v', F', C', runs five kernels on a dense (res+1)^3 grid:
-//   k_adj_p2g      recompute the substep's grid (momentum, mass) from the input state
+//   k_adj_p2g      recompute the substep's grid (momentum, mass) from the input state (k_adj_p2g_warp: float)
 //   k_adj_gridvel  the grid update of every node once: updated velocity (and mass) for the gathers
 //   k_adj_g2p      reverse G2P: per particle, scatter the node-velocity adjoints (float64 adds per
 //                  stencil node) and form dL/dx, dL/dF of the gather and of F' = (I + dt C') F
@@ -18,9 +18,10 @@
 // needs only its variation across a stencil, sum W (g_i - g) (x) dpos_i.  With float node sums,
 // rounding that differs from node to node (in the momentum and in the mass it is divided by) leaves
 // ~1e-7 of the bulk part in that variation, which biased float E- and nu-gradients of 2000-substep
-// rollouts by ~1%.  So the grids are accumulated in float64 for float particle states too, every
-// node contribution formed in float64 from float factors (a product of two floats is exact in
-// double).  For float states the grids the particle kernels read back (updated velocities, node
+// rollouts by ~1%.  So the grids are accumulated in float64 for float particle states too; the
+// contributions of a float state's particles are formed and, within a warp's run of one base node, summed as
+// float pairs hi + lo (see adj_scatter), whose 48 bits keep that variation as float64 terms did.  For float
+// states the grids the particle kernels read back (updated velocities, node
 // adjoints) are then stored as float pairs hi + lo (hi = the float nearest the double, lo = the
 // float nearest the rest): a stencil node's deviation from the stencil's centre node,
 // (hi - hi_c) + (lo - lo_c), is formed in float with the accuracy of the double subtraction rounded
@@ -147,7 +148,10 @@ __device__ __forceinline__ void red_add3(Node4<double>* p, double a, double b, d
 // exact as a pair (one FMA), a sum of pairs keeps about 48 bits, which is what the read-back grids hold,
 // and the float32 pipe has 64 times the rate of the float64 one.  A warp groups its 32 particles by base
 // node and walks them with its lanes as stencil nodes (warp_kernels.cuh); a run's sums reach the grid as
-// one float64 add per node and component.
+// one float64 add per node and component.  A pair overflows where float does (a momentum m v of 1e39 is no number
+// in it, and its node no velocity), and its low part underflows below 1e-30 or so: warps that hold a term outside
+// [1e-27, 1e30] go particle by particle in float64 (adj_scatter_wide).  131,072 particles, 20 steps: 6,515 us a
+// rollout with the check, 6,551 without.
 struct Pair {
   float hi, lo;
 };
@@ -156,6 +160,7 @@ __device__ __forceinline__ Pair pair_sum(float a, float b) {
   const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
   return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
 }
+// a b, exactly (the rounding error of a product by one FMA: Ogita, Rump and Oishi 2005, TwoProductFMA)
 __device__ __forceinline__ Pair pair_prod(float a, float b) {
   const float p = __fmul_rn(a, b);
   return {p, __fmaf_rn(a, b, -p)};
@@ -173,6 +178,40 @@ __device__ __forceinline__ void pair_add(Pair& s, Pair t) {
   s.lo = __fsub_rn(lo, __fsub_rn(s.hi, u.hi));
 }
 
+__device__ __forceinline__ bool pair_holds(float a) {
+  a = fabsf(a);
+  return a == 0.f || (a >= 1e-27f && a <= 1e30f);  // a NaN is not held
+}
+
+// One particle's scatter in float64, as k_adj_p2g and k_adj_g2p do for double states.
+template <bool kReverse>
+__device__ __noinline__ void adj_scatter_wide(const float* rec, int node, int R, float dx, float inv_dx,
+                                              Node4<double>* grid) {
+  constexpr int f0 = kReverse ? 12 : 13;
+  const float fx[3] = {rec[f0], rec[f0 + 1], rec[f0 + 2]};
+  float w[3][3];
+  for (int d = 0; d < 3; ++d) bspline(fx[d], w[d]);
+  for (int o = 0; o < 27; ++o) {
+    const int i = o / 9, j = o / 3 % 3, k = o % 3;
+    Node4<double>* at = grid + node + ((int64_t)i * R + j) * R + k;
+    if constexpr (kReverse) {
+      const double wd = double(w[0][i] * w[1][j] * w[2][k]);
+      const float c4 = 4.f * inv_dx, r[3] = {float(i) - fx[0], float(j) - fx[1], float(k) - fx[2]};
+      double q[3];
+      for (int c = 0; c < 3; ++c)
+        q[c] = wd * (double(rec[c]) + double(c4 * (rec[3 + 3 * c] * r[0] + rec[4 + 3 * c] * r[1] + rec[5 + 3 * c] * r[2])));
+      red_add3(at, q[0], q[1], q[2]);
+    } else {
+      const double wd = double(w[0][i]) * double(w[1][j]) * double(w[2][k]), m = double(rec[0]);
+      const float d[3] = {(float(i) - fx[0]) * dx, (float(j) - fx[1]) * dx, (float(k) - fx[2]) * dx};
+      double q[3];
+      for (int c = 0; c < 3; ++c)
+        q[c] = wd * (m * double(rec[1 + c]) + double(rec[4 + 3 * c] * d[0] + rec[5 + 3 * c] * d[1] + rec[6 + 3 * c] * d[2]));
+      atomic_add4(at, q[0], q[1], q[2], wd * m);
+    }
+  }
+}
+
 // Records: kReverse false (forward P2G): [m, v (3), A (9), fx (3)], a node gets w (m v + A dpos) and w m;
 // true (reverse G2P): [vb (3), Cb (9), fx (3)], a node gets w (vb + c4 Cb r).  The factors are formed as in
 // the float64 kernels below: A dpos, c4 Cb r and (reverse) w in float, the products and sums beyond.
@@ -182,8 +221,25 @@ __device__ __forceinline__ void adj_scatter(WarpRecs<3, float>& wr, const float 
                                             Node4<double>* __restrict__ grid) {
   const unsigned vmask = __ballot_sync(0xffffffffu, node >= 0);
   if (vmask == 0u) return;
-  const int nv = warp_group<3, float>(wr, rec, node, vmask);
   constexpr int NC = kReverse ? 3 : 4, f0 = kReverse ? 12 : 13;
+  bool held = true;
+  if (node >= 0) {
+    const float s = kReverse ? 4.f * kp.inv_dx : kp.dx;  // of a matrix entry
+#pragma unroll
+    for (int i = 0; i < 9; ++i) held = held && pair_holds(rec[f0 - 9 + i] * s);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) held = held && pair_holds(kReverse ? rec[c] : rec[0] * rec[1 + c]);
+    if (!kReverse) held = held && pair_holds(rec[0]);
+  }
+  if (!__all_sync(0xffffffffu, held)) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) wr.rec[lane][i] = rec[i];
+    if (node >= 0) adj_scatter_wide<kReverse>(wr.rec[lane], node, kp.res + 1, kp.dx, kp.inv_dx, grid);
+    __syncwarp();
+    return;
+  }
+  const int nv = warp_group<3, float>(wr, rec, node, vmask);
   const int per = (nv + 2) / 3, l0 = ln.grp * per, l1 = ln.grp < 3 ? min(nv, l0 + per) : 0;
   const int R = kp.res + 1;
   const int64_t RR = (int64_t)R * R;
