@@ -97,7 +97,8 @@ class Batch2D:
         self.ws = (self._wsbuf.data_ptr() + 255) // 256 * 256
         N.call("ffmpm_batch2d_init", tptr, self.nscenes, self.rb, ctypes.c_void_p(self.ws),
                ctypes.c_size_t(self.ws_bytes), ctypes.c_void_p(E._stream_ptr(self.device)))
-        # float32, 4 scenes to 256: 0 to 6 % faster than 256 threads (fewer CTAs at the barriers)
+        # float32: 512 threads mean fewer CTAs at the barriers (10 substeps of 24 scenes: 307 us, 350 with 256; of 256
+        # scenes: 3,044, 3,150); up to 8 scenes of 8,000 particles they are 2 to 5 % slower (156 us, 153)
         self.threads, self.ctas_per_sm = (512 if self.rb == 4 else 256), 0
         self._graph, self._graph_steps = None, 0
 

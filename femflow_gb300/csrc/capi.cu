@@ -62,10 +62,11 @@ bool valid_params(const ffmpm_params* p) {
 }
 
 // One substep (or one phase) on the caller's arrays without a block sort (warp_kernels.cuh): the
-// default outside the deterministic mode and the P2G variants.  Its grid pass reads every node, so a
-// grid that is large against the particle count keeps the sorted form, which visits the touched
-// blocks only.  Both sides at 4 to 17 M nodes: the dense pass costs 9 us at 2.1 M nodes and grows with
-// them (16 bytes a node), the sort and plan it saves 60 to 150 us.
+// default outside the deterministic mode and the P2G variants.  Its grid pass visits every node (9 us at 2.1 M
+// nodes), so a grid that is large against the particle count keeps the sorted form, which visits the touched
+// blocks only.  The line is on the safe side of where the two cross: four substeps of 20,000 particles take 536 us
+// sorted and 478 unsorted on 192^3 (7.2 M nodes), 545 and 683 on 255^3; of 200,000 particles 979 and 636, 1,434 and
+// 877.
 bool unsorted(const ffmpm_params& p, const Layout& L) {
   return !p.deterministic && (p.variant & (kVariantP2GDirect | kVariantP2GLanes)) == 0 &&
          L.nnodes <= std::max<int64_t>(int64_t(1) << 22, 16 * L.n);
@@ -454,7 +455,8 @@ int launch_g2p(const ffmpm_params& p, const Layout& L, const Ws& w, const PView<
 }
 
 // Fused G2P + P2G in the sorted solver: the default outside the deterministic mode and the P2G
-// variants, for runs of two or more substeps (3D blocks of 16 nodes a side keep separate launches).
+// variants, for runs of two or more substeps.  3D blocks of 16 nodes a side keep separate launches, as when the
+// fused kernel's tiles of them did not fit (1,048,576 particles: 312 us a substep, 126 fused, 115 with blocks of 8).
 bool fused(const ffmpm_params& p, const Layout& L, int nsteps) {
   return !p.deterministic && nsteps >= 2 &&
          (p.variant & (kVariantNoFuse | kVariantP2GDirect | kVariantP2GLanes)) == 0 && !(L.dim == 3 && L.bs > 8);
