@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, 2) k_p2g_warp(KParams<T> kp, Geom
 // or, for double particles and few float ones, whose records cost more to write and to wait for than their
 // particles to gather:
 //   k_cell_perm     the particles' indices in their slots, for k_p2g_warp
-// 1,048,576 particles of a random order on 128^3, component-major (GB300): 18 + 5 + 79 + 50 us, where
+// 1,048,576 particles of a random order on 128^3, component-major (GB300): 18 + 5 + 66 + 49 us, where
 // the block sort and the chunked scatter through its permutation took 150 + 305 us (every component
 // of a particle then came from a sector of its own).  k_cell_records is bound by its scattered 64-byte
 // record writes and wants the warps that 80 registers allow (a coarse step of 552 us takes 540 with them),
