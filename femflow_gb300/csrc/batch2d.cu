@@ -209,7 +209,7 @@ __device__ __forceinline__ void widen_box(int* bx, int lo0, int lo1, int hi0, in
 
 // P2G of one particle per lane of a whole warp (every lane calls it) through warp_scatter, the lanes of
 // one scene at a time (a warp nearly always holds one).  256 scenes of 4.4M particles, 10 substeps a call
-// (GB300): 3,266 us, from 4,050 with the nodes' contributions summed by shuffles over runs of lanes;
+// (GB300): 3,037 us (512 threads), from 4,050 with the nodes' contributions summed by shuffles over runs of lanes;
 // bound by instruction issue.  32 warps per SM pay more than the registers they take away: 4,310 us with
 // 16.  Shares of neighbouring particles per warp, instead of the launch-wide stride, take 4,250: every
 // warp then streams rows of its own.  The box of touched nodes of each scene is widened

@@ -2,7 +2,7 @@
 // order, and works on its own (no CTA barrier, no shared tile, no plan).
 //
 //   k_p2g_warp        stress + 3^d-node scatter (three_d/p2g.py:14-80, two_d/p2g.py:11-76)
-//   k_grid_update_dense  momentum -> velocity over every node that received something
+//   k_grid_update_dense  momentum -> velocity at every node
 //   k_g2p_range       gather, advect, F update (three_d/g2p.py:9-59, two_d/g2p.py:5-47)
 //   k_grid_fold_user / k_grid_pack_user  between the workspace grid and a caller's grid arrays
 #pragma once
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(kWarpCta<T>, sizeof(T) == 4 ? 3 : 1) k_g2p_ran
 // cells, its scatter is warp_scatter's (the particles that crossed a cell boundary since the last re-sort
 // join the run of their new cell there).  The grid update visits the blocks the plan touches: a
 // particle whose new stencil may leave them adds the blocks it covers to the list itself.
-// Two cubes of 1,048,576 particles on 128^3 (GB300): 115 us a launch; chunks of 512 particles with a
+// Two cubes of 1,048,576 particles on 128^3 (GB300): 106 us a launch; chunks of 512 particles with a
 // shared-memory tile for each side, an in-chunk counting sort and CTA barriers between the phases took
 // 156.  16,384 particles on 64^3: 13 us a substep against 40 (512 one-warp batches instead of 32 chunks).
 // Bound by instruction issue and the latency of the gathers.
